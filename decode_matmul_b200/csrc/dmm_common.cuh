@@ -402,6 +402,19 @@ __device__ __forceinline__ void bytes_to_half2(uint2 d, uint32_t (&r)[4]) {
     }
 }
 
+// The same as quarters, q / 4: (1024 + u) / 4 - 288 in one fused multiply-add, exact.
+__device__ __forceinline__ void bytes_to_quarters(uint2 d, uint32_t (&r)[4]) {
+    const __half2 quarter = __float2half2_rn(0.25f), bias = __float2half2_rn(-288.0f);
+    const uint32_t magic = 0x64646464u;
+    const uint32_t t[4] = {prmt(d.x, magic, 0x4140u), prmt(d.x, magic, 0x4342u), prmt(d.y, magic, 0x4140u),
+                           prmt(d.y, magic, 0x4342u)};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 h = __hfma2(*reinterpret_cast<const __half2 *>(&t[i]), quarter, bias);
+        r[i] = *reinterpret_cast<const uint32_t *>(&h);
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // Balanced partition of T work items over G CTAs in 32-bit arithmetic (T < 2^31):
 // with a = T / G and b = T % G (computed on the host), the first b CTAs own a + 1 items.
