@@ -17,7 +17,7 @@ X_F16, X_F32, X_F32_SILU_MUL = 0, 1, 2
 STATUS_WAIT_TIMEOUT, STATUS_BAD_CODEBOOK, STATUS_BAD_SMEM = 1, 2, 4
 
 EXPORTS = (
-    "dmm_i8", "dmm_f16", "dmm_f16_fused", "dmm_f16_fused_tp", "dmm_f16_tp_produce", "dmm_f16_tp_consume", "dmm_tp_finalize", "dmm_xrank_barrier", "dmm_xrank_allreduce_add", "dmm_f16_chain", "dmm_f16_noalloc", "dmm_decode", "dmm_workspace_bytes", "dmm_status", "dmm_select_path",
+    "dmm_i8", "dmm_f16", "dmm_f16_fused", "dmm_f16_fused_tp", "dmm_f16_tp_produce", "dmm_f16_tp_consume", "dmm_tp_finalize", "dmm_xrank_barrier", "dmm_xrank_allreduce_add", "dmm_f16_chain", "dmm_f16_sequence", "dmm_f16_noalloc", "dmm_decode", "dmm_workspace_bytes", "dmm_status", "dmm_select_path",
     "dmm_hint_next_weights", "dmm_set_wait_limit_ms", "dmm_launch_count", "dmm_error_string", "dmm_version",
 )
 
@@ -30,6 +30,13 @@ class ChainOp(ctypes.Structure):
     _fields_ = [("x", ctypes.c_void_p), ("x_kind", ctypes.c_int), ("x_ld", ctypes.c_int64), ("x_gap", ctypes.c_int64),
                 ("codes", ctypes.c_void_p), ("scale", ctypes.c_float), ("out", ctypes.c_void_p), ("N", ctypes.c_int64),
                 ("K", ctypes.c_int64), ("zero_ptr", ctypes.c_void_p), ("zero_count", ctypes.c_int64)]
+
+
+class FusedOp(ctypes.Structure):
+    """``dmm_fused_op`` of include/dmm.h."""
+    _fields_ = [("x", ctypes.c_void_p), ("x_kind", ctypes.c_int), ("x_ld", ctypes.c_int64), ("x_gap", ctypes.c_int64),
+                ("codes", ctypes.c_void_p), ("cb16", ctypes.c_void_p), ("scale", ctypes.c_float), ("out", ctypes.c_void_p),
+                ("N", ctypes.c_int64), ("K", ctypes.c_int64), ("zero_ptr", ctypes.c_void_p), ("zero_count", ctypes.c_int64)]
 
 
 def lib() -> ctypes.CDLL:
@@ -68,6 +75,8 @@ def lib() -> ctypes.CDLL:
     L.dmm_xrank_allreduce_add.restype = ci
     L.dmm_f16_chain.argtypes = [vp, ci, vp, i64, ci, cu, vp]
     L.dmm_f16_chain.restype = ci
+    L.dmm_f16_sequence.argtypes = [ctypes.POINTER(FusedOp), ci, i64, ci, cu, vp, i64, i64, vp, sz, vp]
+    L.dmm_f16_sequence.restype = ci
     L.dmm_f16_noalloc.argtypes = [vp, vp, vp, ctypes.c_float, vp, i64, i64, i64, ci, cu, vp]
     L.dmm_f16_noalloc.restype = ci
     L.dmm_decode.argtypes = [vp, vp, ci, vp, i64, i64, ci, ci, vp]

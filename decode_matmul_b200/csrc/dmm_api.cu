@@ -771,6 +771,28 @@ int dmm_status(unsigned *status_out) {
     return 0;
 }
 
+int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_convention, unsigned flags,
+                     const int16_t *next_codes, int64_t next_N, int64_t next_K, void *workspace, size_t workspace_bytes,
+                     void *stream) {
+    if (!ops) return DMM_ERR_NULL;
+    if (n_ops < 1) return DMM_ERR_ARG;
+    for (int i = 0; i < n_ops; ++i) {
+        const dmm_fused_op &op = ops[i];
+        const bool last = i + 1 == n_ops;
+        int rc = last ? dmm_hint_next_weights(next_codes, next_N, next_K)
+                      : dmm_hint_next_weights(ops[i + 1].codes, ops[i + 1].N, ops[i + 1].K);
+        if (rc == 0)
+            rc = dmm_f16_fused(op.x, op.x_kind, op.x_ld, op.x_gap, op.codes, op.cb16, op.scale, op.out, M, op.N, op.K,
+                               sign_convention, DMM_LAYOUT_TILE, DMM_PATH_AUTO, flags, op.zero_ptr, op.zero_count, workspace,
+                               workspace_bytes, stream);
+        if (rc) {
+            t_next_hint = NextHint();
+            return rc;
+        }
+    }
+    return 0;
+}
+
 int dmm_select_path(int64_t M, int64_t N, int64_t K) {
     // Measured on B200: the fp6/fp8-operand kernel (32 batch rows per pass, planes split once by
     // planes_kernel from 4 rows on) beats the fp16-operand one at every batch size.

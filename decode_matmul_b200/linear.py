@@ -372,6 +372,18 @@ class LinearStack:
                                  x_kind=_lib.X_F32_SILU_MUL, x_gap=ffn_loc)]
                 decode_matmul_chain(ops, self.layers[b0]["qkv"].codebook, pdl=True)
             return h
+        from .ops import decode_matmul_sequence, fused_op
+
+        if not tp:
+            # One call into the library per block: the four products of a small model take less time on the GPU
+            # than four calls from Python.  The op list is made anew from the layers on every step.
+            for i, blk in enumerate(self.layers):
+                q, o, gu, dn = blk["qkv"], blk["o"], blk["gate_up"], blk["down"]
+                block = (fused_op(h, q, a, zero=g), fused_op(a, o, h), fused_op(h, gu, g, zero=a),
+                         fused_op(g, dn, h, x_kind=_lib.X_F32_SILU_MUL, x_gap=ffn_loc))
+                nxt = self.layers[i + 1]["qkv"] if i + 1 < len(self.layers) else None
+                decode_matmul_sequence(block, h.shape[0], h.device, next_weights=nxt, workspace=buf["ws"])
+            return h
         from . import ops as _ops
 
         hint = lambda w: _ops.hint_next_weights(w)
@@ -384,21 +396,15 @@ class LinearStack:
             hint(o.codes)
             mm(h, q.codes, q.codebook, q.scale, a, x_kind=_lib.X_F32, zero=g, **kw)
             hint(gu.codes)
-            if tp:
-                mm(a, o.codes, o.codebook, o.scale, po, x_kind=_lib.X_F32, zero=pd, **kw)
-                torch.distributed.all_reduce(po, group=self.group)
-                h.add_(po)
-            else:
-                mm(a, o.codes, o.codebook, o.scale, h, x_kind=_lib.X_F32, **kw)
+            mm(a, o.codes, o.codebook, o.scale, po, x_kind=_lib.X_F32, zero=pd, **kw)
+            torch.distributed.all_reduce(po, group=self.group)
+            h.add_(po)
             hint(dn.codes)
             mm(h, gu.codes, gu.codebook, gu.scale, g, x_kind=_lib.X_F32, zero=a, **kw)
             hint(nxt)
-            if tp:
-                mm(g, dn.codes, dn.codebook, dn.scale, pd, x_kind=_lib.X_F32_SILU_MUL, x_gap=ffn_loc, zero=po, **kw)
-                torch.distributed.all_reduce(pd, group=self.group)
-                h.add_(pd)
-            else:
-                mm(g, dn.codes, dn.codebook, dn.scale, h, x_kind=_lib.X_F32_SILU_MUL, x_gap=ffn_loc, **kw)
+            mm(g, dn.codes, dn.codebook, dn.scale, pd, x_kind=_lib.X_F32_SILU_MUL, x_gap=ffn_loc, zero=po, **kw)
+            torch.distributed.all_reduce(pd, group=self.group)
+            h.add_(pd)
         return h
 
     def _row_parallel(self, lin: DecodeLinear, x16: torch.Tensor, h: torch.Tensor, path: int) -> None:

@@ -6,6 +6,7 @@ include/dmm.h.  Nothing here computes on the CPU and nothing synchronises the de
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 
 import torch
@@ -20,18 +21,33 @@ def _req(cond: bool, msg: str) -> None:
 
 def _check_input(t: torch.Tensor, name: str, dtype: torch.dtype) -> None:
     # same checks as CHECK_INPUT / TORCH_CHECK(scalar_type) in decode_matmul_cuda.cu:16-18,186-188
+    if isinstance(t, torch.Tensor) and t.is_cuda and t.dtype is dtype and t.is_contiguous():
+        return
     _req(isinstance(t, torch.Tensor), f"{name} must be a tensor")
     _req(t.is_cuda, f"{name} must be a CUDA tensor")
     _req(t.is_contiguous(), f"{name} must be contiguous")
     _req(t.dtype == dtype, f"{name} must have dtype {dtype}")
 
 
-def _stream_ptr(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+# A small product takes a few microseconds on the GPU, so what a call costs on the host is what its caller sees:
+# addresses and streams go to the library as plain integers (the argument types are declared in _lib), and the
+# device is only switched when the tensors are on another one than the current.
+def _stream_ptr(device) -> int:
+    index = device.index if isinstance(device, torch.device) else torch.device(device).index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
-def _ptr(t: torch.Tensor) -> ctypes.c_void_p:
-    return ctypes.c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor) -> int:
+    return t.data_ptr()
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def _on_device_of(t: torch.Tensor):
+    """Context in which the tensor's device is the current one."""
+    index = t.get_device()
+    return _SAME_DEVICE if index == torch.cuda.current_device() else torch.cuda.device(index)
 
 
 def decode_matmul_i8(x, weights_compressed, codebook_abs, output=None, *, sign_convention=_lib.SIGN_SLOW,
@@ -50,7 +66,7 @@ def decode_matmul_i8(x, weights_compressed, codebook_abs, output=None, *, sign_c
     _req(x.size(-1) == weights_compressed.size(-1) << 3, "x.size(-1) must equal 8 * weights_compressed.size(-1)")
     M, K = x.shape
     N = weights_compressed.size(0)
-    with torch.cuda.device(x.device):
+    with _on_device_of(x):
         if output is None:
             _req(not accumulate, "accumulate needs an output tensor")
             output = torch.empty((M, N), dtype=torch.int32, device=x.device)
@@ -77,7 +93,7 @@ def decode_matmul_fp16(x, weights_compressed, codebook_fp16, scale=1.0, output=N
     _req(x.size(-1) == weights_compressed.size(-1) << 3, "x.size(-1) must equal 8 * weights_compressed.size(-1)")
     M, K = x.shape
     N = weights_compressed.size(0)
-    with torch.cuda.device(x.device):
+    with _on_device_of(x):
         if output is None:
             _req(not accumulate, "accumulate needs an output tensor")
             output = torch.empty((M, N), dtype=torch.float32, device=x.device)
@@ -122,7 +138,7 @@ def decode_matmul_fused(x, weights_compressed, codebook_fp16, scale, output, *, 
         _check_input(zero, "zero", torch.float32)
     flags = ((_lib.FLAG_ACCUMULATE if accumulate else 0) | (_lib.FLAG_PDL if pdl else 0)
              | (_lib.FLAG_ATOMIC if atomic else 0))
-    with torch.cuda.device(x.device):
+    with _on_device_of(x):
         rc = _lib.lib().dmm_f16_fused(_ptr(x), x_kind, ld, x_gap, _ptr(weights_compressed), _ptr(codebook_fp16),
                                       float(scale), _ptr(output), M, N, K, sign_convention, _lib.LAYOUT_TILE,
                                       _lib.PATH_AUTO, flags, None if zero is None else _ptr(zero),
@@ -131,6 +147,43 @@ def decode_matmul_fused(x, weights_compressed, codebook_fp16, scale, output, *, 
                                       _stream_ptr(x.device))
     _lib.check(rc, "decode_matmul_fused")
     return output
+
+
+def fused_op(x, lin, output, *, x_kind=_lib.X_F32, x_gap=0, zero=None) -> tuple:
+    """One product of :func:`decode_matmul_sequence`: the arguments of :func:`decode_matmul_fused` with ``lin`` a
+    layer (codes, codebook, scale)."""
+    codes, cb = lin.codes, lin.codebook
+    _check_input(x, "x", torch.float16 if x_kind == _lib.X_F16 else torch.float32)
+    _check_input(codes, "weights_compressed", torch.int16)
+    _check_input(cb, "codebook_fp16", torch.float16)
+    _check_input(output, "output", torch.float32)
+    _req(x.dim() == 2 and codes.dim() == 2, "x and weights_compressed must be 2-D")
+    M, ld = x.shape
+    N, k8 = codes.shape
+    _req(ld >= 8 * k8, "x rows are shorter than the reduction length")
+    _req(output.shape == (M, N), "output must have shape [M, N]")
+    if zero is not None:
+        _check_input(zero, "zero", torch.float32)
+    return (x.data_ptr(), x_kind, ld, x_gap, codes.data_ptr(), cb.data_ptr(), lin.scale, output.data_ptr(), N, 8 * k8,
+            None if zero is None else zero.data_ptr(), 0 if zero is None else zero.numel())
+
+
+def decode_matmul_sequence(ops, M, device, *, next_weights=None, sign_convention=_lib.SIGN_SLOW, pdl=True, workspace=None):
+    """Dependent products one after the other (``dmm_f16_sequence``): every op, a :func:`fused_op` over M rows, ADDS
+    its product to its output with atomic adds, and each launch is told which weights the next one streams
+    (``next_weights``: a layer that follows the last op).  One call into the library for all of them."""
+    arr = (_lib.FusedOp * len(ops))(*ops)
+    nxt = (None, 0, 0)
+    if next_weights is not None:
+        n, k8 = next_weights.codes.shape
+        nxt = (next_weights.codes.data_ptr(), n, 8 * k8)
+    flags = _lib.FLAG_ACCUMULATE | _lib.FLAG_ATOMIC | (_lib.FLAG_PDL if pdl else 0)
+    with torch.cuda.device(device):
+        rc = _lib.lib().dmm_f16_sequence(arr, len(ops), M, sign_convention, flags, *nxt,
+                                         None if workspace is None else workspace.data_ptr(),
+                                         0 if workspace is None else workspace.numel() * workspace.element_size(),
+                                         _stream_ptr(device))
+    _lib.check(rc, "decode_matmul_sequence")
 
 
 def workspace_bytes(M: int, N: int, K: int) -> int:
@@ -160,7 +213,7 @@ def decode_matmul_fused_tp(x, weights_compressed, codebook_fp16, scale, peer_out
         _req(move_src.numel() == move_dst.numel(), "move_src and move_dst differ in size")
         n_move = move_src.numel()
     ptrs = (ctypes.c_void_p * len(peer_out_ptrs))(*[int(v) for v in peer_out_ptrs])
-    with torch.cuda.device(x.device):
+    with _on_device_of(x):
         rc = _lib.lib().dmm_f16_fused_tp(_ptr(x), x_kind, ld, x_gap, _ptr(weights_compressed), _ptr(codebook_fp16),
                                          float(scale), ptrs, len(peer_out_ptrs), M, N, K, sign_convention,
                                          _lib.FLAG_PDL if pdl else 0, None if zero is None else _ptr(zero),
@@ -183,7 +236,7 @@ def tp_produce(x, weights_compressed, codebook_fp16, scale, peer_slot_ptrs, peer
     world = len(peer_slot_ptrs)
     slots = (ctypes.c_void_p * world)(*[int(v) for v in peer_slot_ptrs])
     flg = (ctypes.c_void_p * world)(*[int(v) for v in peer_flag_ptrs])
-    with torch.cuda.device(x.device):
+    with _on_device_of(x):
         rc = _lib.lib().dmm_f16_tp_produce(_ptr(x), x_kind, ld, x_gap, _ptr(weights_compressed), _ptr(codebook_fp16),
                                            float(scale), slots, flg, rank, world, M, N, K, sign_convention,
                                            _lib.FLAG_PDL if pdl else 0, _stream_ptr(x.device))
@@ -207,7 +260,7 @@ def tp_consume(h_in, h_out, slots, flags, world, weights_compressed, codebook_fp
     _req(slots.numel() == 2 * world * M * K, "slots must hold [2][world][M * K] floats")
     if zero is not None:
         _check_input(zero, "zero", torch.float32)
-    with torch.cuda.device(h_in.device):
+    with _on_device_of(h_in):
         rc = _lib.lib().dmm_f16_tp_consume(_ptr(h_in), _ptr(h_out), ld, _ptr(slots), _ptr(flags), world, M * K,
                                            _ptr(weights_compressed), _ptr(codebook_fp16), float(scale), _ptr(output), M, N, K,
                                            sign_convention, _lib.FLAG_PDL if pdl else 0, None if zero is None else _ptr(zero),
@@ -219,7 +272,7 @@ def tp_finalize(h_in, h_out, slots, flags, world):
     """``h_out = h_in + the slots of the last epoch`` (``dmm_tp_finalize``)."""
     _check_input(h_in, "h_in", torch.float32)
     _check_input(h_out, "h_out", torch.float32)
-    with torch.cuda.device(h_in.device):
+    with _on_device_of(h_in):
         rc = _lib.lib().dmm_tp_finalize(_ptr(h_in), _ptr(h_out), _ptr(slots), _ptr(flags), world, h_in.numel(),
                                         _stream_ptr(h_in.device))
     _lib.check(rc, "tp_finalize")
@@ -243,7 +296,7 @@ def xrank_allreduce_add(dst, peer_src_ptrs, peer_flag_ptrs, rank, *, zero=None):
     world = len(peer_src_ptrs)
     src = (ctypes.c_void_p * world)(*[int(v) for v in peer_src_ptrs])
     flg = (ctypes.c_void_p * world)(*[int(v) for v in peer_flag_ptrs])
-    with torch.cuda.device(dst.device):
+    with _on_device_of(dst):
         rc = _lib.lib().dmm_xrank_allreduce_add(_ptr(dst), src, None if zero is None else _ptr(zero), dst.numel(), flg,
                                                 rank, world, _stream_ptr(dst.device))
     _lib.check(rc, "xrank_allreduce_add")
@@ -302,7 +355,7 @@ def decode_matmul_fp16_noalloc(x, weights_compressed, codebook_fp16, scale, outp
     N = weights_compressed.size(0)
     _req(tuple(output.shape) == (M, N), "output must have shape [M, N]")
     flags = (_lib.FLAG_ACCUMULATE if accumulate else 0) | (_lib.FLAG_PDL if pdl else 0)
-    with torch.cuda.device(x.device):
+    with _on_device_of(x):
         rc = _lib.lib().dmm_f16_noalloc(_ptr(x), _ptr(weights_compressed), _ptr(codebook_fp16), float(scale),
                                         _ptr(output), M, N, K, sign_convention, flags, _stream_ptr(x.device))
     _lib.check(rc, "decode_matmul_fp16_noalloc")
@@ -318,7 +371,7 @@ def decode_weights(weights_compressed, codebook, *, sign_convention=_lib.SIGN_SL
     _check_input(codebook, "codebook", torch.float16 if is_f16 else torch.int64)
     _req(codebook.numel() == (2048 if is_f16 else 256), "codebook must have 256 entries")
     N, K8 = weights_compressed.shape
-    with torch.cuda.device(weights_compressed.device):
+    with _on_device_of(weights_compressed):
         out = torch.empty((N, K8 * 8), dtype=torch.float16 if is_f16 else torch.int8,
                           device=weights_compressed.device)
         rc = _lib.lib().dmm_decode(_ptr(weights_compressed), _ptr(codebook), int(is_f16), _ptr(out), N, K8 * 8,

@@ -249,6 +249,32 @@ int dmm_f16_chain(const dmm_chain_op *ops, int n_ops, const void *cb16, int64_t 
                   unsigned flags, void *stream);
 
 /*
+ * Dependent products one after the other, one launch each.  (No counterpart in the reference.)
+ *
+ * Every op is one dmm_f16_fused product in the tile layout on the path the library picks, over the same M rows; op
+ * k + 1 may read what op k wrote.  Between two ops the library gives dmm_hint_next_weights for the op that
+ * follows, and next_codes / next_N / next_K (may be null / 0) for what follows the last one.  The
+ * same launches as n_ops calls would make, for programs whose small products take less time on the GPU than
+ * a call from their language does.  flags, workspace and stream as in dmm_f16_fused.  On an error the call
+ * returns at once: the ops before the one that failed have been launched.
+ */
+typedef struct dmm_fused_op {
+    const void *x;        /* activations of this op, see x_kind */
+    int x_kind;           /* DMM_X_F16 / DMM_X_F32 / DMM_X_F32_SILU_MUL */
+    int64_t x_ld, x_gap;  /* as in dmm_f16_fused */
+    const int16_t *codes; /* tiled codes [N, K/8] */
+    const void *cb16;     /* fp16 [256, 8] */
+    float scale;
+    float *out;           /* [M, N] fp32 */
+    int64_t N, K;
+    float *zero_ptr;      /* optional buffer cleared by this op (see dmm_f16_fused) */
+    int64_t zero_count;
+} dmm_fused_op;
+int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_convention, unsigned flags,
+                     const int16_t *next_codes, int64_t next_N, int64_t next_K, void *workspace,
+                     size_t workspace_bytes, void *stream);
+
+/*
  * dmm_f16 for callers that must not allocate.  (No counterpart in the reference.)
  *
  * Some host programs cannot let a library call cudaMalloc on their behalf: a serving
