@@ -10,6 +10,7 @@
 #include "dmm_stream.cuh"
 #include "dmm_umma.cuh"
 #include "dmm_tc.cuh"
+#include "dmm_wide.cuh"
 
 namespace dmm {
 
@@ -52,9 +53,10 @@ static int current_device_state(DeviceState **out) {
     return 0;
 }
 
-// Size of the library's own workspace on first use: tickets for N up to 2^24 (4 MiB), stream-K partials
-// at batch 64 (up to 256 CTAs: 16 MiB) and the activation planes for K up to 2^17 (16 MiB).
-constexpr size_t kDefaultWorkspace = size_t(40) << 20;
+// Size of the library's own workspace on first use: tickets for N up to 2^24 (4 MiB) and behind them either the
+// partial tiles of the wide kernel (148 CTAs, 128 columns: 37 MiB) or stream-K partials at batch 64 (up to
+// 256 CTAs: 16 MiB) and the activation planes for K up to 2^17 (16 MiB).
+constexpr size_t kDefaultWorkspace = size_t(42) << 20;
 
 static size_t ticket_bytes(long long N) {
     const size_t b = static_cast<size_t>(N / 16) * sizeof(unsigned);
@@ -73,6 +75,8 @@ static size_t partial_bytes(long long M, int num_sms) {
 static size_t planes_offset(long long M, long long N, int num_sms) {
     return (ticket_bytes(N) + partial_bytes(M, num_sms) + 255) & ~static_cast<size_t>(255);
 }
+constexpr long long kWideMinBatch = 17;  // from this batch on the wide kernel runs
+
 static size_t workspace_need(long long M, long long N, long long K, int num_sms) {
     return planes_offset(M, N, num_sms) + static_cast<size_t>(K) * 128;
 }
@@ -81,12 +85,13 @@ static size_t workspace_need(long long M, long long N, long long K, int num_sms)
 // grown on demand.  The ticket counters must be zero before the first launch; the
 // library's buffer is cleared when it is (re)allocated, a caller's buffer by the caller.
 static int resolve_workspace(DeviceState *d, long long M, long long N, long long K, void *user, size_t user_bytes,
-                             cudaStream_t stream, void **ws) {
+                             cudaStream_t stream, void **ws, size_t *ws_bytes = nullptr) {
     const size_t need = workspace_need(M, N, K, d->num_sms);
     if (user != nullptr) {
         if (user_bytes < need) return DMM_ERR_WORKSPACE;
         if (reinterpret_cast<uintptr_t>(user) % 256 != 0) return DMM_ERR_ALIGN;
         *ws = user;
+        if (ws_bytes != nullptr) *ws_bytes = user_bytes;
         return 0;
     }
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -110,6 +115,7 @@ static int resolve_workspace(DeviceState *d, long long M, long long N, long long
         d->workspace_bytes = bytes;
     }
     *ws = d->workspace;
+    if (ws_bytes != nullptr) *ws_bytes = d->workspace_bytes;
     return 0;
 }
 
@@ -190,6 +196,59 @@ static int run_stream(int family, const void *x, const void *codes, const void *
 }
 
 
+// Wide fp16-operand kernel (dmm_wide.cuh): every batch row in one launch.  fp32 inputs are rounded to fp16
+// first, up to 64 rows at a time into the part of the workspace that otherwise holds the planes.
+static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, const void *codes, const void *cb16,
+                    float scale, float *out, long long M, long long N, long long K, int sign_convention, unsigned flags,
+                    void *workspace, size_t workspace_bytes, cudaStream_t stream, float *zero_ptr, long long zero_count,
+                    bool fast_layout) {
+    DeviceState *d = nullptr;
+    int rc = current_device_state(&d);
+    if (rc) return rc;
+    void *ws = nullptr;
+    size_t ws_bytes = 0;
+    rc = resolve_workspace(d, M, N, K, workspace, workspace_bytes, stream, &ws, &ws_bytes);
+    if (rc) return rc;
+    const bool pdl = (flags & DMM_FLAG_PDL) != 0;
+    const long long step = x_kind == DMM_X_F16 ? M : 64;
+    t_next_hint = NextHint();  // (a hint is for the next launch only; this kernel has no use for it)
+    for (long long m0 = 0; m0 < M; m0 += step) {
+        const long long rows = M - m0 < step ? M - m0 : step;
+        const uint8_t *xm = reinterpret_cast<const uint8_t *>(x) + static_cast<size_t>(m0) * x_ld * (x_kind == DMM_X_F16 ? 2 : 4);
+        size_t capacity = ws_bytes - ticket_bytes(N);
+        long long ld = x_ld;
+        if (x_kind != DMM_X_F16) {
+            uint8_t *half = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, N, d->num_sms);
+            capacity = planes_offset(M, N, d->num_sms) - ticket_bytes(N);
+            rc = launch_half(xm, x_kind, x_ld, x_gap, static_cast<int>(rows), K, half, pdl, stream);
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+            if (rc) return rc;
+            xm = half;
+            ld = K;
+        }
+        WideParams p = {};
+        p.cb = cb16;
+        p.out = out + static_cast<size_t>(m0) * N;
+        p.tickets = reinterpret_cast<unsigned *>(ws);
+        p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ws) + ticket_bytes(N));
+        p.M = rows;
+        p.N = N;
+        p.scale = scale;
+        p.accumulate = (flags & DMM_FLAG_ACCUMULATE) ? 1 : 0;
+        p.atomic_reduce = (flags & DMM_FLAG_ATOMIC) ? 1 : 0;
+        p.sign_convention = sign_convention;
+        if (m0 == 0) {
+            p.zero_ptr = zero_ptr;
+            p.zero_count = zero_count;
+        }
+        rc = launch_wide(p, xm, ld, codes, K, fast_layout, capacity, static_cast<long long>(ticket_bytes(N) / sizeof(unsigned)), d->num_sms,
+                         pdl, stream);
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        if (rc) return rc;
+    }
+    return 0;
+}
+
 // tcgen05 path: one launch per chunk of 64 batch columns (32 for the fp6/fp8 operand policy,
 // preceded by planes_kernel when the chunk has at least kPlanesMinBatch rows).
 // Tensor-parallel extras of one call (dmm_f16_fused_tp).
@@ -215,6 +274,9 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
     void *ws = nullptr;
     rc = resolve_workspace(d, M, N, K, workspace, workspace_bytes, stream, &ws);
     if (rc) return rc;
+    if (f8 && M >= kWideMinBatch && tp == nullptr)
+        return run_wide(x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K, sign_convention, flags, workspace,
+                        workspace_bytes, stream, zero_ptr, zero_count, fast_layout);
     const long long step = f8 ? 32 : 64;
     const bool pdl = (flags & DMM_FLAG_PDL) != 0;
     for (long long m0 = 0; m0 < M; m0 += step) {
@@ -746,7 +808,12 @@ size_t dmm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
     DeviceState *d = nullptr;
     int sms = 256;
     if (current_device_state(&d) == 0 && d->num_sms > 0) sms = d->num_sms;
-    return workspace_need(M, N, K, sms);
+    size_t need = workspace_need(M, N, K, sms);
+    if (M >= kWideMinBatch) {  // (with less the wide kernel leaves the last tiles whole)
+        const size_t wide = ticket_bytes(N) + wide_partial_bytes(M, sms);
+        if (wide > need) need = wide;
+    }
+    return need;
 }
 
 int dmm_status(unsigned *status_out) {

@@ -165,6 +165,12 @@ __device__ __forceinline__ uint64_t policy_evict_first() {
     return p;
 }
 
+__device__ __forceinline__ uint64_t policy_evict_normal() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+
 // arrives at a named barrier without waiting for it
 __device__ __forceinline__ void named_barrier_arrive(int id, int threads) {
     __threadfence_block();
@@ -237,7 +243,11 @@ constexpr uint32_t kLutBytes = 65536;
 //   kFmtFp6     sign << 5 | |q|, |q| <= 15             (fp6 E2M3 container: the value is q/8,
 //               because E2M3 codes 0..15 are linear: exponent 0 is subnormal m/8, exponent 1 is
 //               (8+m)/8)
-constexpr int kFmtTwos = 0, kFmtOffset = 1, kFmtFp6 = 2;
+//   kFmtHalf    sign << 7 | (|q| - 1) / 2, |q| odd and <= 15: the high byte of the half whose low byte
+//               is 0x80.  Bits 0..10 of a half are linear (subnormals and the first binade), so that
+//               half is (-1)^sign * |q| * 2^-17, exactly: one byte-permute turns two decoded bytes
+//               into a pair of fp16 operands, with no arithmetic.
+constexpr int kFmtTwos = 0, kFmtOffset = 1, kFmtFp6 = 2, kFmtHalf = 3;
 
 // Mask bytes for high code byte h (bit 7 = shift, bits 0..6 = stored signs).
 __host__ __device__ inline uint64_t sign_mask(uint32_t h, int convention, int fmt) {
@@ -255,6 +265,8 @@ __host__ __device__ inline uint64_t sign_mask(uint32_t h, int convention, int fm
         uint64_t b;
         if (fmt == kFmtFp6) {
             b = (sg << 5) | ((sg ^ shift) << 1);
+        } else if (fmt == kFmtHalf) {
+            b = (sg << 7) | (sg ^ shift);
         } else {
             b = (sg ? 0xFCu : 0x00u) ^ (shift ? 0x03u : 0x01u) ^ (fmt == kFmtOffset ? 0x80u : 0x00u);
         }
@@ -271,6 +283,14 @@ __host__ __device__ inline uint32_t sign_mask_fp6_packed(uint32_t h, int convent
     const uint64_t m = sign_mask(h, convention, kFmtFp6);
     const uint32_t lo = static_cast<uint32_t>(m), hi = static_cast<uint32_t>(m >> 32);
     return (lo & 0x22222222u) | ((hi & 0x22222222u) >> 1);
+}
+
+// kFmtHalf masks, packed the same way: weights 0..3 at bits 8j+7 (sign) and 8j (sign ^ shift), weights
+// 4..7 rotated right by four.  (word & 0x81818181) and (rotl(word, 4) & 0x81818181) are the mask words.
+__host__ __device__ inline uint32_t sign_mask_half_packed(uint32_t h, int convention) {
+    const uint64_t m = sign_mask(h, convention, kFmtHalf);
+    const uint32_t lo = static_cast<uint32_t>(m), hi = static_cast<uint32_t>(m >> 32);
+    return (lo & 0x81818181u) | ((hi & 0x81818181u) >> 4) | ((hi & 0x81818181u) << 28);
 }
 
 // Codebook entry e as packed int8 x 8 (= 4 * value), from either table format.  Sets *bad
@@ -296,23 +316,25 @@ __device__ inline uint64_t load_entry(const void *cb, int cb_is_f16, int e, bool
 }
 
 // Entry bytes in the given format.  kFmtFp6: (neg << 5) | ((|c| | 1) ^ (neg << 1)); XOR with
-// the mask byte gives sign = s ^ neg and magnitude |c| + 1 or |c| - 1.
+// the mask byte gives sign = s ^ neg and magnitude |c| + 1 or |c| - 1.  kFmtHalf: the same with
+// (magnitude - 1) / 2 in bits 0..2 and the sign in bit 7.
 __device__ inline uint64_t format_entry(uint64_t v, int fmt, bool *bad) {
-    if (fmt != kFmtFp6) return v;
+    if (fmt != kFmtFp6 && fmt != kFmtHalf) return v;
     uint64_t r = 0;
     for (int i = 0; i < 8; ++i) {
         const int c = static_cast<int8_t>((v >> (8 * i)) & 0xFFu);
         const uint32_t neg = c < 0 ? 1u : 0u;
         const uint32_t mag = static_cast<uint32_t>(c < 0 ? -c : c);
         if (mag > 14u) *bad = true;
-        r |= static_cast<uint64_t>((neg << 5) | (((mag | 1u) ^ (neg << 1)) & 0x1Fu)) << (8 * i);
+        const uint32_t fp6 = ((mag | 1u) ^ (neg << 1)) & 0x1Fu;
+        r |= static_cast<uint64_t>(fmt == kFmtFp6 ? (neg << 5) | fp6 : (neg << 7) | ((fp6 >> 1) & 7u)) << (8 * i);
     }
     return r;
 }
 
 // Fills the table; every thread of the group calls it (tid in [0, nthreads)).
 // Returns true when this thread saw an entry that the XOR decode cannot represent.
-// packed_mask: store the kFmtFp6 masks as 32 replicas of the packed 32-bit word.
+// packed_mask: store the kFmtFp6 or kFmtHalf masks as 32 replicas of the packed 32-bit word.
 // Work item i < 512: entry row i & 255, half i >> 8 (0 = table entry, 1 = sign mask), so that the
 // lanes of a warp all take the same branch.
 // pre: the fp16 entry of thread tid (tid < 256), loaded earlier with lut_prefetch so that
@@ -331,7 +353,8 @@ __device__ inline bool lut_fill(uint32_t lut_addr, const void *cb, int cb_is_f16
         const int part = i >> 8;
         uint4 rep;
         if (part == 1 && packed_mask) {
-            const uint32_t w = sign_mask_fp6_packed(static_cast<uint32_t>(e), convention);
+            const uint32_t w = fmt == kFmtHalf ? sign_mask_half_packed(static_cast<uint32_t>(e), convention)
+                                               : sign_mask_fp6_packed(static_cast<uint32_t>(e), convention);
             rep = make_uint4(w, w, w, w);
         } else {
             const uint64_t v = part == 0 ? format_entry(load_entry(cb, cb_is_f16, e, &bad, pre), fmt, &bad)
@@ -374,6 +397,19 @@ __device__ __forceinline__ uint2 decode8_fp6(uint32_t word, const LutLane &l) {
     uint32_t m2;  // m << 1 as an integer multiply-add: the FMA pipe is idle, the integer ALU is not
     asm("mad.lo.u32 %0, %1, %2, 0;" : "=r"(m2) : "r"(m), "r"(l.two));
     return make_uint2(e.x ^ (m & 0x22222222u), e.y ^ (m2 & 0x22222222u));
+}
+
+// kFmtHalf with packed masks: the eight weights of a code as four words of two halves, q * 2^-17.
+template <int which>
+__device__ __forceinline__ uint4 decode8_half(uint32_t word, const LutLane &l) {
+    constexpr uint32_t sel_idx = which == 0 ? 0x7604u : 0x7624u;
+    constexpr uint32_t sel_hi = which == 0 ? 0x7614u : 0x7634u;
+    const uint2 e = lds64(prmt(word, l.entry_c, sel_idx));
+    const uint32_t m = lds32(prmt(word, l.mask_c, sel_hi));
+    const uint32_t lo = e.x ^ (m & 0x81818181u);
+    const uint32_t hi = e.y ^ (__funnelshift_l(m, m, 4) & 0x81818181u);
+    constexpr uint32_t low = 0x80808080u;  // the constant low byte of every half
+    return make_uint4(prmt(lo, low, 0x1404u), prmt(lo, low, 0x3424u), prmt(hi, low, 0x1404u), prmt(hi, low, 0x3424u));
 }
 
 // Decodes the code in half `which` (0 = low 16 bits, 1 = high) of `word`: 8 packed bytes.

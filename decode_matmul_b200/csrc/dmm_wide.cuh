@@ -1,0 +1,691 @@
+// Wide decode-matmul kernel of the fp16 family: fp16 operands, up to 128 batch columns per pass over
+// the codes.  (The kernels of dmm_umma.cuh split the activations into four fp8 planes, which is the
+// better trade while the product is a weight stream; from some ten batch rows on the planes cost more
+// tensor-core time and shared-memory traffic than the fp16 operands cost in the decode.)
+//
+// Data path.  A decoder thread turns its codes into fp16 weights in registers -- two table look-ups, two
+// XORs and four byte-permutes per eight weights, no arithmetic: the table holds the HIGH byte of the half
+// q * 2^-17 (kFmtHalf in dmm_common.cuh) -- and writes them into tensor memory as the A operand of
+// tcgen05.mma kind::f16 (M = 128, K = 16).  The activations are the B operand: TMA copies 64 k of every
+// batch row into shared memory with the 128-byte swizzle and the MMA reads them as they lie there.
+// Accumulators are fp32 in TMEM; the epilogue multiplies by 2^15 (2^17, and 1/4 for quarter units) and scale.
+//
+// Why 256 output rows x up to 128 columns per CTA.  One 16-byte piece of the code stream holds the codes of
+// rows g and g + 8, so a thread decodes for two MMA tiles (256 rows).  Per 2 KiB tile of codes (256 rows x
+// 32 k) and NB columns an SM needs
+//   tensor pipe      4 MMAs of max(44, NB / 2) cycles, and every tcgen05.commit costs as much as a small MMA:
+//                    one commit per 64 k serves the weight slots and the activation stage alike
+//   shared memory    96 table look-ups + 32 codes in and out + 1.5 NB
+//   integer ALU      9 operations per code, 144 cycles
+//
+// Accuracy.  kind::f16 truncates when it adds to the accumulator: over a chain of n MMAs the sums shrink by a part
+// in 2^24 or so per MMA (measured against 64 bits: 4.2e-7 after 64, 9.7e-7 after 128, 2.6e-5 after 1792).
+// The fp8 planes stay at 7.5e-7 whatever the length.  So a chain is cut after at most kWChain units of 64 k (80
+// MMAs, 5e-7): the decoder warps add the accumulators to fp32 sums in registers (rounded to nearest) and the
+// next chain starts from zero.  That is why a column tile ends at 128: its sums are 64 registers per thread.
+// Up to 64 columns there are two accumulator sets, so the next chain starts while the last one is read.
+//
+// Work split.  A tile of output is (256 rows, NB columns); its reduction is cut into units of 64 k.  While
+// there are more tiles than CTAs every CTA computes whole tiles; the units of the tiles that remain are
+// split evenly and contiguously over the CTAs (stream-K), partial tiles go through the workspace and
+// the last CTA to arrive (ticket) sums them in a fixed order, or straight into `out` with atomic adds
+// (DMM_FLAG_ATOMIC).  No CTA waits for another.  With too little workspace for the partials the remaining
+// tiles are computed whole.
+//
+// Warp roles (20 warps):
+//   0..15  decoders, four groups; group q decodes the k-tiles (32 k) whose CTA-wide number is q mod 4
+//          into its own kNA weight slots in TMEM.  Warp wq of a group owns TMEM lanes 32wq..32wq+31.
+//          They also build the look-up table, keep the sums and run the epilogue.  A chain is read, and
+//          a segment written out, only after the first k-tiles of the next one are decoded, so that the
+//          tensor core always has work.
+//   16     MMA issuer (one for both MMA tiles: the summation order is fixed); allocates the tensor memory
+//   17     TMA producer of the codes (one thread), 18 of the activations (the only thread whose loads
+//          depend on the previous kernel of the stream); warp 18 also clears zero_ptr.
+// Every wait is bounded (mbar_wait).
+#pragma once
+#include "dmm_umma.cuh"
+
+namespace dmm {
+
+constexpr int kWDecWarps = 16, kWMmaWarp = 16, kWCodeWarp = 17, kWXWarp = 18;
+constexpr int kWThreads = 20 * 32;              // (warp 19 completes the last warpgroup and has no work)
+constexpr int kWMaxCols = 128;
+constexpr int kWChain = 20;                     // units (of four MMAs per accumulator) before the sums leave the tensor core
+constexpr int kWDone = 16;                      // ring of "unit done" barriers
+constexpr int kWRing = 14;                      // code units in flight (even: a decoder group meets every second one)
+constexpr uint32_t kWUnitBytes = 16 * 2 * 128;  // codes of 64 k of 16 strips
+constexpr uint32_t kWBarBytes = 2048;
+constexpr uint32_t kWPreBytes = kWBarBytes + kWRing * kWUnitBytes;
+constexpr uint32_t kWXBytes = 100 * 1024;       // activation stages, behind the table
+constexpr int kWMaxStages = 16;
+constexpr uint32_t kWDynBytes = 0x10000u - 0x400u + kLutBytes + kWXBytes;
+static_assert(kWPreBytes <= 0x10000u - 0x400u, "the code ring does not fit below the table");
+static_assert(kWDynBytes <= 232448u, "shared memory plan exceeds the per-CTA limit");
+static_assert(kWXBytes / (kWMaxCols * 128u) >= 3, "too few activation stages");
+
+struct WideParams {
+    const void *cb;     // fp16 [256, 8]
+    float *out;         // [M, N]
+    float *partials;    // workspace [grid][2][NB * 256]
+    unsigned *tickets;  // workspace, one per split tile, zero between launches
+    long long M, N;
+    float scale;
+    int accumulate, atomic_reduce, sign_convention;
+    int nb;             // batch columns per tile: a multiple of 16, at most kWMaxCols
+    int units;          // units of 64 k per tile
+    int sst;            // super-tiles (256 output rows)
+    int whole;          // whole tiles per CTA before the split ones
+    int split_grid;     // CTAs that share the split tiles (0: none are left)
+    Part32 part;        // split units per CTA
+    int stages;         // activation stages
+    float *zero_ptr;    // optional: buffer this kernel clears on its way
+    long long zero_count;
+    unsigned dyn_smem_bytes;
+};
+struct WideArgs {
+    WideParams p;
+    CUtensorMap codes_map, x_map;
+};
+
+// kCols: columns the variant is built for (32, 64 or 128).  Two accumulator sets while the sums and the weight
+// slots leave room; kNA weight slots per decoder group fill the rest of the tensor memory.
+template <int kCols>
+struct WidePlan {
+    static constexpr int kSets = kCols <= 64 ? 2 : 1;
+    static constexpr int kNA = kCols <= 32 ? 3 : 2;
+    static constexpr uint32_t kSetCols = 2 * kCols;
+    static constexpr uint32_t kSlotCols = 32;  // [MMA tile][16 columns = 32 k x 2 bytes]
+    static constexpr uint32_t kACol = kUTmemCols - 4 * kNA * kSlotCols;
+    static_assert(kSets * kSetCols <= kACol, "TMEM plan exceeds 512 columns");
+    static constexpr int kBarCode = 0;                            // [kWRing] TMA completion
+    static constexpr int kBarEmpty = kBarCode + kWRing;           // [kWRing] the eight warps that read the unit
+    static constexpr int kBarFull = kBarEmpty + kWRing;           // [4 kNA] the group's four warps
+    static constexpr int kBarXFull = kBarFull + 4 * kNA;          // [kWMaxStages] TMA completion
+    static constexpr int kBarDone = kBarXFull + kWMaxStages;      // [kWDone] commit: unit u (mod kWDone) has been multiplied,
+                                                                  // its weight slots and activation stage are free
+    static constexpr int kBarDReady = kBarDone + kWDone;          // [kSets] commit: the chain is complete
+    static constexpr int kBarDFree = kBarDReady + kSets;          // [kSets] every decoder warp has read it
+    static constexpr int kBarCount = kBarDFree + kSets;
+    static_assert(kWDone >= kWMaxStages && kWDone >= 2 * kNA + 2, "a Done barrier must not be reused before it is waited for");
+    static_assert(kBarCount * 8 + 64 <= kWBarBytes && kBarCount <= 96, "barrier block too small");
+};
+
+__device__ __forceinline__ void tma_load_2d_plain(uint32_t dst, const void *tmap, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(tmap), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+
+// D[tmem] (+)= A[tmem] * B[smem descriptor], kind::f16, the descriptor as two 32-bit words
+__device__ __forceinline__ void mma_ts_f16_lh(uint32_t d, uint32_t a, uint32_t desc_lo, uint32_t desc_hi, uint32_t idesc,
+                                              uint32_t acc) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 bd;\nsetp.ne.b32 p, %5, 0;\nmov.b64 bd, {%2, %3};\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n}\n" ::"r"(d),
+        "r"(a), "r"(desc_lo), "r"(desc_hi), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+// Segments (parts of a tile) of one CTA, in order: first its whole tiles, then what its range of the
+// split units covers.
+struct WideSeg {
+    int ss, nt;    // super-tile and column tile
+    int u0, u1;    // units
+    int split;     // index of the split tile, -1 for a whole tile
+};
+struct WideWork {
+    int whole, grid, cta, sst, units, i0, i1;
+    __device__ __forceinline__ WideWork(const WideParams &p) {
+        whole = p.whole;
+        grid = static_cast<int>(gridDim.x);
+        cta = static_cast<int>(blockIdx.x);
+        sst = p.sst;
+        units = p.units;
+        i0 = i1 = 0;
+        if (cta < p.split_grid) {
+            i0 = part32_begin(p.part, cta);
+            i1 = part32_begin(p.part, cta + 1);
+        }
+    }
+    __device__ __forceinline__ int count() const { return whole + (i1 > i0 ? (i1 - 1) / units - i0 / units + 1 : 0); }
+    __device__ __forceinline__ WideSeg get(int seg) const {
+        WideSeg s;
+        int tile;
+        if (seg < whole) {
+            tile = seg * grid + cta;
+            s.u0 = 0;
+            s.u1 = units;
+            s.split = -1;
+        } else {
+            s.split = i0 / units + (seg - whole);
+            tile = whole * grid + s.split;
+            const int a = s.split * units;
+            s.u0 = i0 > a ? i0 - a : 0;
+            s.u1 = i1 < a + units ? i1 - a : units;
+        }
+        s.nt = tile / sst;
+        s.ss = tile - s.nt * sst;
+        return s;
+    }
+};
+
+// Chains of one segment: its units cut into equal parts of at most kWChain.
+__device__ __forceinline__ int wide_chains(int units) { return (units + kWChain - 1) / kWChain; }
+
+template <int kCols, bool kFast>
+__global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constant__ WideArgs args) {
+    using Plan = WidePlan<kCols>;
+    constexpr int kNA = Plan::kNA, kSets = Plan::kSets;
+    const WideParams &p = args.p;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    const uint32_t base = smem_u32(smem_raw);
+    const uint32_t lut_addr = (base + kWPreBytes + 0xFFFFu) & ~0xFFFFu;
+    const uint32_t ring_addr = base + kWBarBytes;
+    const uint32_t x_addr = lut_addr + kLutBytes;  // 1024-byte aligned, as the swizzle needs
+    volatile int *flags = reinterpret_cast<volatile int *>(smem_raw + Plan::kBarCount * 8);  // [0]=failed [1]=last
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem_raw + Plan::kBarCount * 8 + 16);
+    auto bar = [&](int i) -> uint32_t { return base + 8u * static_cast<uint32_t>(i); };
+
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const uint4 cb_pre = lut_prefetch(p.cb, tid);
+    if (x_addr + kWXBytes > base + p.dyn_smem_bytes) {  // uniform over the grid
+        if (tid == 0) raise_status(DMM_STATUS_BAD_SMEM);
+        return;
+    }
+    const WideWork work(p);
+    const int nseg = work.count();
+    const uint32_t stage_b = static_cast<uint32_t>(p.nb) * 128u;
+
+    // ---- set-up: the decoders build the table; the other warps initialise the barriers, allocate TMEM and go on
+    // (the code stream starts flowing meanwhile), arriving on the decoders' barrier only ----
+    bool bad_cb = false;
+    if (warp < kWDecWarps) {
+        bad_cb = lut_fill(lut_addr, p.cb, 1, p.sign_convention, kFmtHalf, tid, kWDecWarps * 32, true, &cb_pre);
+        named_barrier(4, kWThreads);
+    } else {
+        const int bt = tid - kWDecWarps * 32;
+        if (bt < Plan::kBarCount) {
+            uint32_t count = 1;                                                     // TMA completion, commit
+            if (bt >= Plan::kBarEmpty && bt < Plan::kBarFull) count = 8;
+            if (bt >= Plan::kBarFull && bt < Plan::kBarXFull) count = 4;
+            if (bt >= Plan::kBarDFree) count = kWDecWarps;
+            mbar_init(bar(bt), count);
+            if (bt == 0) {
+                flags[0] = 0;
+                flags[1] = 0;
+            }
+            fence_mbar_init();
+        }
+        if (warp == kWMmaWarp) tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), kUTmemCols);
+        fence_async_smem();
+        tc_fence_before();
+        named_barrier(3, kWThreads - kWDecWarps * 32);
+        named_barrier_arrive(4, kWThreads);
+    }
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    grid_dep_launch();
+
+    // 128 columns: the decoders need 64 registers for the sums.  Of the 96 x 640 registers of the launch they take
+    // 112 x 512 and leave 32 x 128 to the other warpgroup, which is all of them.
+    if (kCols > 64 && warp >= kWDecWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    if (warp < kWDecWarps) {
+        // =============================== decoders ===============================
+        if (kCols > 64) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+        const int q = warp >> 2, wq = warp & 3;
+        if (bad_cb) raise_status(DMM_STATUS_BAD_CODEBOOK);
+        const LutLane ll = lut_lane(lut_addr, lane, true);
+        const uint32_t tlane = tmem + (static_cast<uint32_t>(wq * 32) << 16);
+        const uint32_t abase = tlane + Plan::kACol + static_cast<uint32_t>(q * kNA) * Plan::kSlotCols;
+        const int par = q >> 1, ki = q & 1;  // this group decodes k-tile ki of the units of parity par
+        const uint32_t lane_off = (wq * 4 + (lane >> 3)) * 256 + ki * 128 + (lane & 7) * 16;
+        const int mt = q >> 1;               // its part of the sums: MMA tile mt, column groups of parity q % 2
+        int rs = par;            // ring slot of my next unit, and the parity of its barrier
+        uint32_t cpar = 0;
+        int buf = 0;             // my next weight slot
+        constexpr int kGroups = kCols / 32;  // groups of 16 columns whose sums this thread keeps
+        float sum[kGroups][16];
+
+        int un = 0;              // units of this CTA before the current chain
+        int chains = 0;          // chains of this CTA so far (the accumulator set and the phase of its barriers)
+        WideSeg s = {}, prev = {};
+        bool pending = false, prev_first = false, prev_last = false;  // a chain that has not been read yet
+        for (int seg = 0, c = 0, nc = 0;;) {
+            // next chain: c of nc of segment seg
+            const bool more = seg < nseg;
+            int u_end = un, first_part = un;
+            if (more) {
+                if (c == 0) {
+                    s = work.get(seg);
+                    nc = wide_chains(s.u1 - s.u0);
+                }
+                const int len = s.u1 - s.u0;
+                u_end = un + (len * (c + 1) / nc - len * c / nc);
+                // what is decoded before the previous chain is read: as many k-tiles as there are weight slots
+                first_part = pending ? (un + 2 * kNA < u_end ? un + 2 * kNA : u_end) : u_end;
+            }
+            int u = un + ((un ^ par) & 1);
+            for (int part = 0; part < 2; ++part) {
+                const int stop = part == 0 ? first_part : u_end;
+                for (; u < stop; u += 2) {
+                    mbar_wait(bar(Plan::kBarCode + rs), cpar, flags);
+                    const uint32_t slot_addr = ring_addr + static_cast<uint32_t>(rs) * kWUnitBytes;
+                    uint4 cw;
+                    if constexpr (kFast)
+                        cw = fetch_fast_ktile(slot_addr, 2, wq, lane, ki);
+                    else
+                        cw = lds128(slot_addr + lane_off);
+                    const uint32_t w[4] = {cw.x, cw.y, cw.z, cw.w};
+                    // the slot held unit u - 2 kNA
+                    const int v = u - 2 * kNA;
+                    const uint32_t acol = abase + static_cast<uint32_t>(buf) * Plan::kSlotCols;
+                    uint32_t r[16];
+                    if constexpr (kCols <= 64) {
+                        uint32_t r1[16];
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) {
+                            const uint4 d0 = decode8_half<0>(w[t], ll), d1 = decode8_half<1>(w[t], ll);
+                            r[4 * t] = d0.x; r[4 * t + 1] = d0.y; r[4 * t + 2] = d0.z; r[4 * t + 3] = d0.w;
+                            r1[4 * t] = d1.x; r1[4 * t + 1] = d1.y; r1[4 * t + 2] = d1.z; r1[4 * t + 3] = d1.w;
+                        }
+                        if (v >= 0) mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
+                        tc_fence_after();
+                        tmem_st16(acol, r);
+                        tmem_st16(acol + 16, r1);
+                    } else {  // one MMA tile after the other: the sums leave no registers for both
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) {
+                            const uint4 d = decode8_half<0>(w[t], ll);
+                            r[4 * t] = d.x; r[4 * t + 1] = d.y; r[4 * t + 2] = d.z; r[4 * t + 3] = d.w;
+                        }
+                        if (v >= 0) mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
+                        tc_fence_after();
+                        tmem_st16(acol, r);
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) {
+                            const uint4 d = decode8_half<1>(w[t], ll);
+                            r[4 * t] = d.x; r[4 * t + 1] = d.y; r[4 * t + 2] = d.z; r[4 * t + 3] = d.w;
+                        }
+                        tmem_st16(acol + 16, r);
+                    }
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(bar(Plan::kBarFull + q * kNA + buf));
+                        mbar_arrive(bar(Plan::kBarEmpty + rs));
+                    }
+                    if (++buf == kNA) buf = 0;
+                    rs += 2;
+                    if (rs >= kWRing) {
+                        rs -= kWRing;
+                        cpar ^= 1u;
+                    }
+                }
+                if (part == 0 && pending) {
+                    // ---------------- the previous chain: its accumulators into the sums ----------------
+                    const int set = (chains - 1) & (kSets - 1);
+                    mbar_wait(bar(Plan::kBarDReady + set), ((chains - 1) / kSets) & 1, flags);
+                    tc_fence_after();
+                    const uint32_t dcol = tlane + static_cast<uint32_t>(set) * Plan::kSetCols + static_cast<uint32_t>(mt * kCols);
+#pragma unroll
+                    for (int g = 0; g < kGroups; ++g) {
+                        const int b0 = 32 * g + 16 * (q & 1);
+                        if (b0 < p.nb) {
+                            uint32_t a[16];
+                            __syncwarp();
+                            tmem_ld16(dcol + static_cast<uint32_t>(b0), a);
+                            tmem_wait_ld(a);
+#pragma unroll
+                            for (int e = 0; e < 16; ++e)
+                                sum[g][e] = prev_first ? __uint_as_float(a[e]) : sum[g][e] + __uint_as_float(a[e]);
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(Plan::kBarDFree + set));
+
+                    if (prev_last) {
+                        // ---------------- epilogue of the previous segment ----------------
+                        const int trow = wq * 32 + lane;
+                        const long long n = kFast ? static_cast<long long>(prev.ss) * 256 + 32 * (4 * mt + wq) + lane
+                                                  : (static_cast<long long>(prev.ss) * 16 + wq * 4 + (lane >> 3)) * 16 + 8 * mt + (lane & 7);
+                        const long long m0 = static_cast<long long>(prev.nt) * p.nb;
+                        const int mcols = static_cast<int>(p.M - m0 < p.nb ? p.M - m0 : p.nb);  // columns that are batch rows
+                        const bool row_ok = n < p.N;
+                        float *const out = p.out + m0 * p.N + n;
+                        const bool full = prev.u0 == 0 && prev.u1 == p.units;
+                        // (2^15 first: exact, and the product with scale then rounds and overflows as scale * sum does)
+                        auto put = [&](int b, float v) {
+                            float *const o = out + b * p.N;
+                            const float r = v * 32768.0f * p.scale;
+                            *o = p.accumulate ? *o + r : r;
+                        };
+                        if (p.atomic_reduce || full) {
+                            if (row_ok) {
+#pragma unroll
+                                for (int g = 0; g < kGroups; ++g) {
+                                    const int b0 = 32 * g + 16 * (q & 1);
+#pragma unroll
+                                    for (int e = 0; e < 16; ++e) {
+                                        if (b0 + e >= mcols) continue;
+                                        if (p.atomic_reduce)
+                                            atomicAdd(out + (b0 + e) * p.N, sum[g][e] * 32768.0f * p.scale);
+                                        else
+                                            put(b0 + e, sum[g][e]);
+                                    }
+                                }
+                            }
+                        } else {
+                            const long long part_sz = static_cast<long long>(p.nb) * 256;
+                            float *const mine = p.partials + (2ll * work.cta + (prev.u0 > 0 ? 0 : 1)) * part_sz +
+                                                static_cast<long long>(mt) * p.nb * 128 + trow;
+#pragma unroll
+                            for (int g = 0; g < kGroups; ++g) {
+                                const int b0 = 32 * g + 16 * (q & 1);
+#pragma unroll
+                                for (int e = 0; e < 16; ++e)
+                                    if (b0 + e < mcols) __stcg(mine + (b0 + e) * 128, sum[g][e]);
+                            }
+                            __threadfence();
+                            named_barrier(1, kWDecWarps * 32);
+                            const int a = prev.split * p.units;
+                            const int c_lo = part32_owner(p.part, a), c_hi = part32_owner(p.part, a + p.units - 1);
+                            if (tid == 0) {
+                                const unsigned old = atomicAdd(p.tickets + prev.split, 1u);
+                                const int last = old == static_cast<unsigned>(c_hi - c_lo);
+                                if (last) p.tickets[prev.split] = 0;
+                                flags[1] = last;
+                            }
+                            named_barrier(1, kWDecWarps * 32);
+                            if (flags[1] != 0) {
+                                __threadfence();
+#pragma unroll
+                                for (int g = 0; g < kGroups; ++g) {
+                                    const int b0 = 32 * g + 16 * (q & 1);
+                                    if (b0 < mcols) {
+                                        float v[16];
+#pragma unroll
+                                        for (int e = 0; e < 16; ++e) v[e] = 0.f;
+                                        for (int cc = c_lo; cc <= c_hi; ++cc) {  // fixed summation order, sixteen loads in flight
+                                            const float *src = p.partials + (2ll * cc + (part32_begin(p.part, cc) > a ? 0 : 1)) * part_sz +
+                                                               (static_cast<long long>(mt) * p.nb + b0) * 128 + trow;
+                                            float l[16];
+#pragma unroll
+                                            for (int e = 0; e < 16; ++e) l[e] = b0 + e < mcols ? __ldcg(src + e * 128) : 0.f;
+#pragma unroll
+                                            for (int e = 0; e < 16; ++e) v[e] += l[e];
+                                        }
+                                        if (row_ok) {
+#pragma unroll
+                                            for (int e = 0; e < 16; ++e)
+                                                if (b0 + e < mcols) put(b0 + e, v[e]);
+                                        }
+                                    }
+                                }
+                            }
+                            named_barrier(1, kWDecWarps * 32);  // flags[1] is reused by the next segment
+                        }
+                    }
+                }
+            }
+            if (!more) break;
+            un = u_end;
+            ++chains;
+            pending = true;
+            prev = s;
+            prev_first = c == 0;
+            prev_last = c + 1 == nc;
+            if (++c == nc) {
+                c = 0;
+                ++seg;
+            }
+        }
+    } else if (warp == kWMmaWarp) {
+        // =============================== MMA issuer ===============================
+        const bool leader = elect_one();
+        // D fp32 (1 at bit 4), A and B fp16 (0), N >> 3 at bit 17, M >> 4 at bit 24
+        const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(p.nb >> 3) << 17) | ((128u >> 4) << 24);
+        // 128-byte swizzle (2 at bit 61), 8-row groups 1024 bytes apart, version 1 at bit 46
+        const uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+        const uint32_t a0 = tmem + Plan::kACol;
+        const uint32_t x16 = ((x_addr >> 4) & 0x3FFFu) | (1u << 16), stage16 = stage_b >> 4;
+        int xs = 0, buf = 0, un = 0, chains = 0;
+        uint32_t xpar = 0, fullpar = 0;
+        for (int seg = 0; seg < nseg; ++seg) {
+            const WideSeg s = work.get(seg);
+            const int len = s.u1 - s.u0, nc = wide_chains(len);
+            for (int c = 0; c < nc; ++c, ++chains) {
+                const int set = chains & (kSets - 1);
+                if (chains >= kSets) {
+                    mbar_wait(bar(Plan::kBarDFree + set), ((chains / kSets) - 1) & 1, flags);
+                    tc_fence_after();
+                }
+                const uint32_t d = tmem + static_cast<uint32_t>(set) * Plan::kSetCols;
+                uint32_t acc = 0u;
+                const int n = len * (c + 1) / nc - len * c / nc;
+                for (int u = 0; u < n; ++u, ++un) {
+                    mbar_wait(bar(Plan::kBarXFull + xs), xpar, flags);
+                    const uint32_t xlo = x16 + static_cast<uint32_t>(xs) * stage16;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int sl = ((un & 1) * 2 + i) * kNA + buf;  // the unit's parity and k-tile name the decoder group
+                        mbar_wait(bar(Plan::kBarFull + sl), fullpar, flags);
+                        tc_fence_after();
+                        if (leader) {
+                            const uint32_t a = a0 + static_cast<uint32_t>(sl) * Plan::kSlotCols;
+                            mma_ts_f16_lh(d, a, xlo + i * 4, desc_hi, idesc, acc);
+                            mma_ts_f16_lh(d + kCols, a + 16, xlo + i * 4, desc_hi, idesc, acc);
+                            mma_ts_f16_lh(d, a + 8, xlo + i * 4 + 2, desc_hi, idesc, 1u);
+                            mma_ts_f16_lh(d + kCols, a + 24, xlo + i * 4 + 2, desc_hi, idesc, 1u);
+                        }
+                        acc = 1u;
+                    }
+                    if (leader) tc_commit(bar(Plan::kBarDone + (un & (kWDone - 1))));
+                    if (++xs == p.stages) {
+                        xs = 0;
+                        xpar ^= 1u;
+                    }
+                    if ((un & 1) != 0 && ++buf == kNA) {
+                        buf = 0;
+                        fullpar ^= 1u;
+                    }
+                }
+                if (leader) tc_commit(bar(Plan::kBarDReady + set));
+            }
+        }
+    } else if (warp == kWCodeWarp) {
+        // =============================== TMA producer: codes ===============================
+        if (lane == 0) {
+            // codes that no other column tile reads again need not stay in L2
+            const uint64_t policy = p.M <= p.nb ? policy_evict_first() : policy_evict_normal();
+            int rs = 0;
+            uint32_t par = 1;
+            uint32_t n = 0;
+            for (int seg = 0; seg < nseg; ++seg) {
+                const WideSeg s = work.get(seg);
+                for (int u = s.u0; u < s.u1; ++u, ++n) {
+                    if (n >= kWRing) mbar_wait(bar(Plan::kBarEmpty + rs), par, flags);
+                    const uint32_t b = bar(Plan::kBarCode + rs);
+                    mbar_arrive_expect_tx(b, kWUnitBytes);
+                    // always the full box: words past the row or strips past N read as zero
+                    tma_load_2d(ring_addr + static_cast<uint32_t>(rs) * kWUnitBytes, &args.codes_map, kFast ? u * 128 : u * 64,
+                                kFast ? s.ss * 8 : s.ss * 16, b, policy);
+                    if (++rs == kWRing) {
+                        rs = 0;
+                        par ^= 1u;
+                    }
+                }
+            }
+            if (flags[0]) {  // a wait gave up: let the loads in flight land before the CTA exits
+                for (uint32_t e = 0; e < kWRing && e < n; ++e) {
+                    const uint32_t i = n - 1 - e;
+                    mbar_wait_limit(bar(Plan::kBarCode + static_cast<int>(i % kWRing)), (i / kWRing) & 1, 20ll * 1000 * 1000);
+                }
+            }
+        }
+    } else if (warp == kWXWarp) {
+        // ============================ TMA producer: activations ============================
+        grid_dep_wait();
+        asm volatile("fence.proxy.async;" ::: "memory");  // x may be the previous kernel's plain stores
+        if (lane == 0) {
+            int xs = 0;
+            uint32_t n = 0;
+            const uint32_t ns = static_cast<uint32_t>(p.stages);
+            for (int seg = 0; seg < nseg; ++seg) {
+                const WideSeg s = work.get(seg);
+                for (int u = s.u0; u < s.u1; ++u, ++n) {
+                    if (n >= ns) {  // the stage held unit n - ns
+                        const uint32_t v = n - ns;
+                        mbar_wait(bar(Plan::kBarDone + static_cast<int>(v & (kWDone - 1))), (v / kWDone) & 1, flags);
+                    }
+                    const uint32_t b = bar(Plan::kBarXFull + xs);
+                    mbar_arrive_expect_tx(b, stage_b);
+                    // k past the row reads as zero (the weights decoded there are finite), and so do rows past M
+                    tma_load_2d_plain(x_addr + static_cast<uint32_t>(xs) * stage_b, &args.x_map, u * 64, s.nt * p.nb, b);
+                    if (++xs == p.stages) xs = 0;
+                }
+            }
+            if (flags[0]) {
+                for (uint32_t e = 0; e < ns && e < n; ++e) {
+                    const uint32_t i = n - 1 - e;
+                    mbar_wait_limit(bar(Plan::kBarXFull + static_cast<int>(i % ns)), (i / ns) & 1, 20ll * 1000 * 1000);
+                }
+            }
+        } else if (p.zero_ptr != nullptr) {  // a later kernel will accumulate into it
+            for (long long i = static_cast<long long>(blockIdx.x) * 31 + lane - 1; i < p.zero_count;
+                 i += static_cast<long long>(gridDim.x) * 31)
+                p.zero_ptr[i] = 0.f;
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kWMmaWarp) tmem_dealloc(tmem, kUTmemCols);
+}
+
+// Batch columns per tile: as few equal column tiles as fit, in steps of 16.
+inline int wide_cols(long long M) {
+    const long long nt = (M + kWMaxCols - 1) / kWMaxCols;
+    return static_cast<int>(((M + nt - 1) / nt + 15) / 16 * 16);
+}
+// Workspace bytes of the partial tiles.
+inline size_t wide_partial_bytes(long long M, int num_sms) {
+    return static_cast<size_t>(num_sms) * 2 * static_cast<size_t>(wide_cols(M)) * 256 * sizeof(float);
+}
+
+// fp32 activations (plain, or silu(gate) * up) rounded to fp16 once per call: [M, K] fp16 for the TMA of
+// wide_kernel.  One thread per eight values.
+__global__ void __launch_bounds__(128) half_kernel(const void *x, int x_mode, long long x_ld, long long x_gap, int M,
+                                                   long long K, __half *out) {
+    grid_dep_wait();
+    grid_dep_launch();
+    const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const long long per_row = K / 8;
+    if (idx >= M * per_row) return;
+    const int row = static_cast<int>(idx / per_row);
+    const long long k0 = (idx - row * per_row) * 8;
+    uint32_t h[4];
+    load_piece(x, x_mode, x_ld, x_gap, row, k0, h);
+    *reinterpret_cast<uint4 *>(out + row * K + k0) = make_uint4(h[0], h[1], h[2], h[3]);
+}
+inline int launch_half(const void *x, int x_mode, long long x_ld, long long x_gap, int M, long long K, void *out, bool pdl,
+                       cudaStream_t stream) {
+    const long long pieces = M * (K / 8);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>((pieces + 127) / 128));
+    cfg.blockDim = dim3(128);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, half_kernel, x, x_mode, x_ld, x_gap, M, K, reinterpret_cast<__half *>(out));
+}
+
+// Tensor map of the activations: fp16 [M, K], rows x_ld elements apart, box 64 k x nb rows, 128-byte swizzle.
+inline int make_x_map(CUtensorMap *map, const void *x, long long M, long long K, long long x_ld, int nb) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (fn == nullptr) return cudaErrorNotSupported;
+    const cuuint64_t gdim[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(M)};
+    const cuuint64_t gstride[1] = {static_cast<cuuint64_t>(x_ld) * 2};
+    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(nb)};
+    const cuuint32_t estride[2] = {1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(x), gdim, gstride, box, estride,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : static_cast<int>(cudaErrorInvalidValue);
+}
+
+template <int kCols, bool kFast>
+inline int launch_wide_as(WideArgs &args, unsigned grid, bool pdl, cudaStream_t stream) {
+    auto kernel = wide_kernel<kCols, kFast>;
+    // the shared-memory attribute is set once per kernel variant and device, not on every launch
+    static std::atomic<unsigned long long> attr_done;
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev >= 64 || !((attr_done.load(std::memory_order_acquire) >> dev) & 1ull)) {
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kWDynBytes));
+        if (err != cudaSuccess) return err;
+        if (dev < 64) attr_done.fetch_or(1ull << dev, std::memory_order_release);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kWThreads);
+    cfg.dynamicSmemBytes = kWDynBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
+// p carries cb, out, partials, tickets, M, N, scale, flags, sign convention and the buffer to clear; x is fp16
+// [M, K] with rows x_ld elements apart.  partial_capacity: bytes of workspace behind p.partials; n_tickets: counters at p.tickets.
+inline int launch_wide(WideParams p, const void *x, long long x_ld, const void *codes, long long K, bool fast_layout,
+                       size_t partial_capacity, long long n_tickets, int num_sms, bool pdl, cudaStream_t stream) {
+    WideArgs args = {};
+    p.nb = wide_cols(p.M);
+    p.units = static_cast<int>((K + 63) / 64);
+    p.sst = static_cast<int>((p.N + 255) / 256);
+    const long long tiles = static_cast<long long>(p.sst) * ((p.M + p.nb - 1) / p.nb);
+    if (tiles * p.units >= (1ll << 31)) return DMM_ERR_SHAPE;
+    long long whole = tiles / num_sms, rest = tiles - whole * num_sms;
+    long long grid = whole > 0 ? num_sms : 0;
+    const bool can_split = p.atomic_reduce || (partial_capacity >= wide_partial_bytes(p.M, num_sms) && rest <= n_tickets);
+    if (rest > 0) {
+        // at least two units per CTA: below that the pipeline's fill costs more than the split gains
+        long long parts = can_split ? rest * p.units / 2 : rest;
+        if (parts < rest) parts = rest;
+        if (parts > num_sms) parts = num_sms;
+        p.split_grid = static_cast<int>(parts);
+        if (!can_split) {  // one whole tile each
+            p.part.a = p.units;
+            p.part.b = 0;
+        } else {
+            p.part.a = static_cast<int>(rest * p.units / parts);
+            p.part.b = static_cast<int>(rest * p.units % parts);
+        }
+        if (parts > grid) grid = parts;
+    }
+    p.whole = static_cast<int>(whole);
+    const int fit = static_cast<int>(kWXBytes / (static_cast<uint32_t>(p.nb) * 128u));
+    p.stages = fit < kWMaxStages ? fit : kWMaxStages;
+    p.dyn_smem_bytes = kWDynBytes;
+    args.p = p;
+    int rc = make_codes_map(&args.codes_map, codes, p.N, K, 2, fast_layout);
+    if (rc) return rc;
+    rc = make_x_map(&args.x_map, x, p.M, K, x_ld, p.nb);
+    if (rc) return rc;
+    const unsigned g = static_cast<unsigned>(grid);
+    if (p.nb <= 32) return fast_layout ? launch_wide_as<32, true>(args, g, pdl, stream) : launch_wide_as<32, false>(args, g, pdl, stream);
+    if (p.nb <= 64) return fast_layout ? launch_wide_as<64, true>(args, g, pdl, stream) : launch_wide_as<64, false>(args, g, pdl, stream);
+    return fast_layout ? launch_wide_as<128, true>(args, g, pdl, stream) : launch_wide_as<128, false>(args, g, pdl, stream);
+}
+
+}  // namespace dmm

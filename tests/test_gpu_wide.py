@@ -1,0 +1,133 @@
+"""The wide fp16-operand kernel (17 batch rows and more) against the CPU oracle, at the sizes where its tiles,
+units and splits end.  Needs a B200."""
+import numpy as np
+import pytest
+import torch
+
+import decode_matmul_b200 as dmm
+from decode_matmul_b200 import _lib
+from oracle import dmm_oracle as o
+
+pytestmark = pytest.mark.gpu
+
+# Products of a half and an odd multiple of 1/4 are exact in fp32, so the only error is that of the fp32 sums: with
+# K terms each addition is off by at most 2^-23 of the running sum (tensor cores may truncate), and the running
+# sums of random terms stay within a few times the result's root mean square.  K <= 2048 terms in steps of 16
+# are 128 additions; their errors add like a random walk with drift: 128 * 2^-23 = 1.5e-5 at the very worst.
+REL = 1.5e-5
+
+
+def _dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.fixture(autouse=True)
+def _status_clean():
+    yield
+    assert dmm.status() == 0, "a kernel raised the device status word"
+
+
+def _case(M, N, K, seed=0, codebook="e8p"):
+    rng = np.random.default_rng(M * 1000003 + N * 101 + K + seed)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    codes = rng.integers(-32768, 32768, size=(N, K // 8)).astype(np.int16)
+    cb16 = o.cb64_to_cb16(np.ascontiguousarray(o.build_codebook_abs())) if codebook == "e8p" else o.synthetic_codebook(42)
+    return x, codes, cb16
+
+
+def _want(x, codes, cb16, convention=None):
+    w = o.decode_weights_f16(codes, cb16) if convention is None else o.decode_weights_f16(codes, cb16, convention)
+    return x.astype(np.float64) @ w.astype(np.float64).T
+
+
+def _rel(y, want):
+    return np.linalg.norm(y.astype(np.float64) - want) / np.linalg.norm(want)
+
+
+# rows around every column-tile size (64, 128, 192 and their multiples), N around 256, K around 64 and 128
+SHAPES = [(17, 16, 32), (17, 272, 64), (31, 256, 96), (32, 528, 1056), (33, 240, 2048), (48, 4096, 544), (64, 512, 512),
+          (65, 512, 160), (128, 272, 1024), (129, 256, 2048), (192, 320, 128), (193, 528, 1056), (333, 1024, 512),
+          (400, 16, 96), (577, 4096, 128), (1000, 9472, 64)]
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+def test_shapes(M, N, K):
+    x, codes, cb16 = _case(M, N, K, codebook="e8p" if M % 2 else "synthetic")
+    want = _want(x, codes, cb16)
+    tiled, cb = _dev(o.tile_pack(codes)), _dev(cb16)
+    first = None
+    for _ in range(2):  # the second call checks that the workspace counters were reset
+        y = dmm.decode_matmul_fp16(_dev(x), tiled, cb).cpu().numpy()
+        assert _rel(y, want) <= REL
+        assert first is None or np.array_equal(first, y), "the summation order must be fixed"
+        first = y
+
+
+@pytest.mark.parametrize("M", [24, 100, 200])
+def test_fast_layout_and_convention(M):
+    x, codes, cb16 = _case(M, 544, 1056, 1)
+    want = _want(x, codes, cb16, o.SIGN_FAST)
+    y = dmm.decode_matmul_fp16(_dev(x), dmm.fast_pack(_dev(codes)), _dev(cb16), sign_convention=_lib.SIGN_FAST,
+                               layout=_lib.LAYOUT_FAST).cpu().numpy()
+    assert _rel(y, want) <= REL
+
+
+@pytest.mark.parametrize("M", [20, 70, 333])
+@pytest.mark.parametrize("atomic", [False, True])
+def test_accumulate_and_scale(M, atomic):
+    x, codes, cb16 = _case(M, 768, 1024, 2)
+    base = np.random.default_rng(3).standard_normal((M, 768)).astype(np.float32)
+    out = _dev(base)
+    y = dmm.decode_matmul_fp16(_dev(x), _dev(o.tile_pack(codes)), _dev(cb16), 0.125, out, accumulate=True, atomic=atomic)
+    assert y.data_ptr() == out.data_ptr()
+    assert _rel(y.cpu().numpy(), base + 0.125 * _want(x, codes, cb16)) <= REL
+
+
+@pytest.mark.parametrize("M", [17, 64, 65, 150])
+@pytest.mark.parametrize("silu", [False, True])
+def test_fp32_inputs_and_clearing(M, silu):
+    """fp32 activations are rounded to fp16 first, as the narrower kernels do; `zero` is cleared on the way."""
+    N, K = 288, 1056
+    x, codes, cb16 = _case(M, N, K, 4)
+    rng = np.random.default_rng(5)
+    xf = rng.standard_normal((M, 2 * K if silu else K)).astype(np.float32)
+    xt = torch.from_numpy(xf)
+    half = (torch.nn.functional.silu(xt[:, :K]) * xt[:, K:] if silu else xt).to(torch.float16).numpy()
+    zero = torch.full((1000,), 7.0, device="cuda")
+    out = torch.zeros((M, N), device="cuda")
+    dmm.decode_matmul_fused(_dev(xf), _dev(o.tile_pack(codes)), _dev(cb16), 1.0, out,
+                            x_kind=_lib.X_F32_SILU_MUL if silu else _lib.X_F32, x_gap=K if silu else 0, accumulate=True,
+                            atomic=True, zero=zero)
+    # silu in the kernel uses the fast exponential: its rounding to half can differ by an ulp here and there
+    assert _rel(out.cpu().numpy(), _want(half, codes, cb16)) <= (1e-4 if silu else REL)
+    assert float(zero.abs().max()) == 0.0
+
+
+def test_small_workspace_leaves_the_tiles_whole():
+    """A caller's workspace that only fits the narrower kernels is accepted, as is one of the full size."""
+    M, N, K = 333, 512, 1024
+    x, codes, cb16 = _case(M, N, K, 6)
+    want = _want(x, codes, cb16)
+    full = dmm.workspace_bytes(M, N, K)
+    for size in (full, full - 256, dmm.workspace_bytes(64, N, K) if dmm.workspace_bytes(64, N, K) < full else full):
+        ws = torch.zeros((size,), dtype=torch.uint8, device="cuda")
+        out = torch.empty((M, N), device="cuda")
+        dmm.decode_matmul_fused(_dev(x), _dev(o.tile_pack(codes)), _dev(cb16), 1.0, out, x_kind=_lib.X_F16, workspace=ws)
+        assert _rel(out.cpu().numpy(), want) <= REL
+
+
+@pytest.mark.parametrize("M", [32, 192])
+def test_extreme_activations(M):
+    """Largest and smallest halves: the weights are 2^-17 units inside the kernel, the result must not show it."""
+    x, codes, cb16 = _case(M, 256, 256, 7)
+    rng = np.random.default_rng(8)
+    x[:, :] = rng.choice(np.array([65504, -65504, 6e-8, -6e-8, 0.0, 1.0], dtype=np.float16), size=x.shape)
+    x[3, :] = np.float16(6e-8)
+    want = _want(x, codes, cb16)
+    y = dmm.decode_matmul_fp16(_dev(x), _dev(o.tile_pack(codes)), _dev(cb16)).cpu().numpy()
+    assert _rel(y, want) <= REL
+    assert _rel(y[3], want[3]) <= REL
+    x[5, 7] = np.float16("inf")
+    x[6, 9] = np.float16("nan")
+    y = dmm.decode_matmul_fp16(_dev(x), _dev(o.tile_pack(codes)), _dev(cb16)).cpu().numpy()
+    assert np.all(~np.isfinite(y[5])) and np.all(np.isnan(y[6])) and np.all(np.isfinite(np.delete(y, [5, 6], axis=0)))
