@@ -196,8 +196,8 @@ static int run_stream(int family, const void *x, const void *codes, const void *
 }
 
 
-// Wide fp16-operand kernel (dmm_wide.cuh): every batch row in one launch.  fp32 inputs are rounded to fp16
-// first, up to 64 rows at a time into the part of the workspace that otherwise holds the planes.
+// Wide fp16-operand kernel (dmm_wide.cuh): every batch row in one launch.  fp32 inputs of more than kWConvRows rows
+// are rounded to fp16 first, up to 64 rows at a time into the part of the workspace that otherwise holds the planes.
 static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, const void *codes, const void *cb16,
                     float scale, float *out, long long M, long long N, long long K, int sign_convention, unsigned flags,
                     void *workspace, size_t workspace_bytes, cudaStream_t stream, float *zero_ptr, long long zero_count,
@@ -217,7 +217,8 @@ static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, 
         const uint8_t *xm = reinterpret_cast<const uint8_t *>(x) + static_cast<size_t>(m0) * x_ld * (x_kind == DMM_X_F16 ? 2 : 4);
         size_t capacity = ws_bytes - ticket_bytes(N);
         long long ld = x_ld;
-        if (x_kind != DMM_X_F16) {
+        int mode = x_kind;
+        if (x_kind != DMM_X_F16 && rows > kWConvRows) {
             uint8_t *half = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, N, d->num_sms);
             capacity = planes_offset(M, N, d->num_sms) - ticket_bytes(N);
             rc = launch_half(xm, x_kind, x_ld, x_gap, static_cast<int>(rows), K, half, pdl, stream);
@@ -225,6 +226,7 @@ static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, 
             if (rc) return rc;
             xm = half;
             ld = K;
+            mode = DMM_X_F16;
         }
         WideParams p = {};
         p.cb = cb16;
@@ -241,7 +243,7 @@ static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, 
             p.zero_ptr = zero_ptr;
             p.zero_count = zero_count;
         }
-        rc = launch_wide(p, xm, ld, codes, K, fast_layout, capacity, static_cast<long long>(ticket_bytes(N) / sizeof(unsigned)), d->num_sms,
+        rc = launch_wide(p, xm, mode, ld, x_gap, codes, K, fast_layout, capacity, static_cast<long long>(ticket_bytes(N) / sizeof(unsigned)), d->num_sms,
                          pdl, stream);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (rc) return rc;

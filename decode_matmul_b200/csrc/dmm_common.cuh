@@ -101,6 +101,23 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// One look at a phase, without suspending.  A look takes some 140 cycles while the shared-memory pipe is busy,
+// whether the phase is complete or not: a warp on the critical path looks ahead of time and does other work
+// meanwhile, and calls mbar_wait only when the phase was not complete then.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Waits (bounded, like mbar_wait) until a counter in global memory that other CTAs of the same
 // grid increment has reached `target`.  Only legal when all those CTAs are resident together.
 __device__ __forceinline__ void grid_wait(const unsigned *counter, unsigned target, volatile int *failed) {

@@ -431,6 +431,21 @@ __device__ __forceinline__ void load_piece_sum(const float *h_in, float *h_out, 
     }
 }
 
+// Eight fp32 activations (or, for kXSiluMul, silu(a) * b) rounded to four packed half2 words.
+__device__ __forceinline__ void pack_piece(int x_mode, const float4 (&a)[2], const float4 (&b)[2], uint32_t (&h)[4]) {
+    float f[8] = {a[0].x, a[0].y, a[0].z, a[0].w, a[1].x, a[1].y, a[1].z, a[1].w};
+    if (x_mode == kXSiluMul) {
+        const float g[8] = {b[0].x, b[0].y, b[0].z, b[0].w, b[1].x, b[1].y, b[1].z, b[1].w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = __fdividef(f[j], 1.0f + __expf(-f[j])) * g[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const __half2 hh = __floats2half2_rn(f[2 * j], f[2 * j + 1]);
+        h[j] = *reinterpret_cast<const uint32_t *>(&hh);
+    }
+}
+
 // Eight consecutive activations of one row as four packed half2 words, from any input kind.
 __device__ __forceinline__ void load_piece(const void *xp, int x_mode, long long x_ld, long long x_gap, int row,
                                            long long k0, uint32_t (&h)[4]) {
@@ -441,21 +456,13 @@ __device__ __forceinline__ void load_piece(const void *xp, int x_mode, long long
         return;
     }
     const float *xf = reinterpret_cast<const float *>(xp) + row * x_ld + k0;
-    const float4 a0 = __ldcg(reinterpret_cast<const float4 *>(xf));
-    const float4 a1 = __ldcg(reinterpret_cast<const float4 *>(xf + 4));
-    float f[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    const float4 a[2] = {__ldcg(reinterpret_cast<const float4 *>(xf)), __ldcg(reinterpret_cast<const float4 *>(xf + 4))};
+    float4 b[2];
     if (x_mode == kXSiluMul) {
-        const float4 b0 = __ldcg(reinterpret_cast<const float4 *>(xf + x_gap));
-        const float4 b1 = __ldcg(reinterpret_cast<const float4 *>(xf + x_gap + 4));
-        const float g[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = __fdividef(f[j], 1.0f + __expf(-f[j])) * g[j];
+        b[0] = __ldcg(reinterpret_cast<const float4 *>(xf + x_gap));
+        b[1] = __ldcg(reinterpret_cast<const float4 *>(xf + x_gap + 4));
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const __half2 hh = __floats2half2_rn(f[2 * j], f[2 * j + 1]);
-        h[j] = *reinterpret_cast<const uint32_t *>(&hh);
-    }
+    pack_piece(x_mode, a, b, h);
 }
 
 // Plane `pl` of a piece = the top byte of each half (an E5M2 number: truncation of the half);

@@ -13,55 +13,61 @@
 // Why 256 output rows x up to 128 columns per CTA.  One 16-byte piece of the code stream holds the codes of
 // rows g and g + 8, so a thread decodes for two MMA tiles (256 rows).  Per 2 KiB tile of codes (256 rows x
 // 32 k) and NB columns an SM needs
-//   tensor pipe      4 MMAs of max(44, NB / 2) cycles, and every tcgen05.commit costs as much as a small MMA:
-//                    one commit per 64 k serves the weight slots and the activation stage alike
+//   tensor pipe      4 MMAs of NB / 2 cycles
 //   shared memory    96 table look-ups + 32 codes in and out + 1.5 NB
-//   integer ALU      9 operations per code, 144 cycles
+//   integer ALU      9 operations per code and some 40 around them: 180 cycles
+// Measured 255 cycles per tile up to 32 columns (the decoders: latency of their waits and look-ups, ALU 70 % busy) and
+// 330 .. 350 at 128.  28672 x 8192: 34.6 us at 16 rows, 36.3 at 32 (the fp8 planes: 35.7, 48.1), 42.5 at 64, 62 at
+// 128; 2048 x 8192 x 28672 863 us (1.1 PFLOP/s; 3455 as passes of 32 rows).
 //
 // Accuracy.  kind::f16 truncates when it adds to the accumulator: over a chain of n MMAs the sums shrink by a part
 // in 2^24 or so per MMA (measured against 64 bits: 4.2e-7 after 64, 9.7e-7 after 128, 2.6e-5 after 1792).
-// The fp8 planes stay at 7.5e-7 whatever the length.  So a chain is cut after at most kWChain units of 64 k (80
-// MMAs, 5e-7): the decoder warps add the accumulators to fp32 sums in registers (rounded to nearest) and the
+// The fp8 planes stay at 7.5e-7 whatever the length.  So a chain is cut after at most kWChain units of 128 k (88
+// MMAs, 6.2e-7): the decoder warps add the accumulators to fp32 sums in registers (rounded to nearest) and the
 // next chain starts from zero.  That is why a column tile ends at 128: its sums are 64 registers per thread.
 // Up to 64 columns there are two accumulator sets, so the next chain starts while the last one is read.
 //
-// Work split.  A tile of output is (256 rows, NB columns); its reduction is cut into units of 64 k.  While
+// Work split.  A tile of output is (256 rows, NB columns); its reduction is cut into units of 128 k.  While
 // there are more tiles than CTAs every CTA computes whole tiles; the units of the tiles that remain are
 // split evenly and contiguously over the CTAs (stream-K), partial tiles go through the workspace and
 // the last CTA to arrive (ticket) sums them in a fixed order, or straight into `out` with atomic adds
 // (DMM_FLAG_ATOMIC).  No CTA waits for another.  With too little workspace for the partials the remaining
 // tiles are computed whole.
 //
-// Warp roles (20 warps):
-//   0..15  decoders, four groups; group q decodes the k-tiles (32 k) whose CTA-wide number is q mod 4
-//          into its own kNA weight slots in TMEM.  Warp wq of a group owns TMEM lanes 32wq..32wq+31.
-//          They also build the look-up table, keep the sums and run the epilogue.  A chain is read, and
-//          a segment written out, only after the first k-tiles of the next one are decoded, so that the
-//          tensor core always has work.
-//   16     MMA issuer (one for both MMA tiles: the summation order is fixed); allocates the tensor memory
-//   17     TMA producer of the codes (one thread), 18 of the activations (the only thread whose loads
-//          depend on the previous kernel of the stream); warp 18 also clears zero_ptr.
+// Warp roles (20 warps, 24 with kConv):
+//   0..15  decoders, four groups; group q decodes the half units (64 k) whose CTA-wide number is q mod 4 into
+//          its weight slot in TMEM.  Warp wq of a group owns TMEM lanes 32wq..32wq+31.  They also build the
+//          look-up table, keep the sums and run the epilogue.  A chain is read, and a segment written out,
+//          only after the first units of the next one are decoded, so that the tensor core always has work.
+//   16,17  MMA issuers, one per MMA tile (each accumulator has one issuer: the summation order is fixed);
+//          warp 16 allocates the tensor memory
+//   18     TMA producer of the codes (one thread), 19 of the activations (the only thread whose loads
+//          depend on the previous kernel of the stream); warp 19 also clears zero_ptr.
+//   kConv (fp32 activations, plain or silu(gate) * up, up to 32 batch rows): warps 19..22 load the activations
+//          of every fourth half unit each, round them to fp16 and store them as the TMA would have; warp 23 clears
+//          zero_ptr.  A kernel that converts them beforehand costs a launch per product, more than this.
 // Every wait is bounded (mbar_wait).
 #pragma once
 #include "dmm_umma.cuh"
 
 namespace dmm {
 
-constexpr int kWDecWarps = 16, kWMmaWarp = 16, kWCodeWarp = 17, kWXWarp = 18;
-constexpr int kWThreads = 20 * 32;              // (warp 19 completes the last warpgroup and has no work)
+constexpr int kWDecWarps = 16, kWMmaWarp = 16, kWCodeWarp = 18, kWXWarp = 19;
+constexpr int kWThreads = 20 * 32;
+constexpr int kWConvThreads = 24 * 32, kWLoaders = 4, kWClearWarp = 23;
+constexpr int kWConvRows = 32;                  // batch rows up to which the kernel converts fp32 activations itself
 constexpr int kWMaxCols = 128;
-constexpr int kWChain = 20;                     // units (of four MMAs per accumulator) before the sums leave the tensor core
-constexpr int kWDone = 16;                      // ring of "unit done" barriers
-constexpr int kWRing = 14;                      // code units in flight (even: a decoder group meets every second one)
-constexpr uint32_t kWUnitBytes = 16 * 2 * 128;  // codes of 64 k of 16 strips
+constexpr int kWChain = 11;                     // units (of eight MMAs per accumulator) before the sums leave the tensor core
+constexpr int kWDone = 16;                      // ring of "half unit done" barriers
+constexpr uint32_t kWUnitBytes = 16 * 4 * 128;  // codes of a unit: 128 k of 16 strips, 512 contiguous bytes of each
+constexpr int kWRingPre = 6;                    // ring slots below the table
 constexpr uint32_t kWBarBytes = 2048;
-constexpr uint32_t kWPreBytes = kWBarBytes + kWRing * kWUnitBytes;
-constexpr uint32_t kWXBytes = 100 * 1024;       // activation stages, behind the table
+constexpr uint32_t kWPreBytes = kWBarBytes + kWRingPre * kWUnitBytes;
+constexpr uint32_t kWPostBytes = 100 * 1024;    // behind the table: activation stages and further ring slots
 constexpr int kWMaxStages = 16;
-constexpr uint32_t kWDynBytes = 0x10000u - 0x400u + kLutBytes + kWXBytes;
+constexpr uint32_t kWDynBytes = 0x10000u - 0x400u + kLutBytes + kWPostBytes;
 static_assert(kWPreBytes <= 0x10000u - 0x400u, "the code ring does not fit below the table");
 static_assert(kWDynBytes <= 232448u, "shared memory plan exceeds the per-CTA limit");
-static_assert(kWXBytes / (kWMaxCols * 128u) >= 3, "too few activation stages");
 
 struct WideParams {
     const void *cb;     // fp16 [256, 8]
@@ -72,7 +78,7 @@ struct WideParams {
     float scale;
     int accumulate, atomic_reduce, sign_convention;
     int nb;             // batch columns per tile: a multiple of 16, at most kWMaxCols
-    int units;          // units of 64 k per tile
+    int units;          // units of 128 k per tile
     int sst;            // super-tiles (256 output rows)
     int whole;          // whole tiles per CTA before the split ones
     int split_grid;     // CTAs that share the split tiles (0: none are left)
@@ -80,6 +86,9 @@ struct WideParams {
     int stages;         // activation stages
     float *zero_ptr;    // optional: buffer this kernel clears on its way
     long long zero_count;
+    const void *x;      // kConv: fp32 activations as in UmmaParams
+    int x_mode;
+    long long x_ld, x_gap, K;
     unsigned dyn_smem_bytes;
 };
 struct WideArgs {
@@ -87,26 +96,29 @@ struct WideArgs {
     CUtensorMap codes_map, x_map;
 };
 
-// kCols: columns the variant is built for (32, 64 or 128).  Two accumulator sets while the sums and the weight
-// slots leave room; kNA weight slots per decoder group fill the rest of the tensor memory.
+// kCols: columns the variant is built for (32, 64 or 128).  Two accumulator sets while the sums leave room.
 template <int kCols>
 struct WidePlan {
     static constexpr int kSets = kCols <= 64 ? 2 : 1;
-    static constexpr int kNA = kCols <= 32 ? 3 : 2;
+    // Code units in flight.  The stream needs some 96 KiB in flight per SM; 128 columns leave room for half of
+    // that beside the activations, and stream at less than half the rate.
+    static constexpr int kRing = kCols <= 64 ? 2 * kWRingPre : kWRingPre;
+    static constexpr uint32_t kXBytes = kWPostBytes - (kRing - kWRingPre) * kWUnitBytes;  // activation stages
+    static_assert(kRing % 2 == 0 && kXBytes / (kCols * 128u) >= 4, "too few activation stages");
     static constexpr uint32_t kSetCols = 2 * kCols;
-    static constexpr uint32_t kSlotCols = 32;  // [MMA tile][16 columns = 32 k x 2 bytes]
-    static constexpr uint32_t kACol = kUTmemCols - 4 * kNA * kSlotCols;
+    static constexpr uint32_t kSlotCols = 64;  // [k-tile][MMA tile][16 columns = 32 k x 2 bytes]
+    static constexpr uint32_t kACol = kUTmemCols - 4 * kSlotCols;
     static_assert(kSets * kSetCols <= kACol, "TMEM plan exceeds 512 columns");
-    static constexpr int kBarCode = 0;                            // [kWRing] TMA completion
-    static constexpr int kBarEmpty = kBarCode + kWRing;           // [kWRing] the eight warps that read the unit
-    static constexpr int kBarFull = kBarEmpty + kWRing;           // [4 kNA] the group's four warps
-    static constexpr int kBarXFull = kBarFull + 4 * kNA;          // [kWMaxStages] TMA completion
-    static constexpr int kBarDone = kBarXFull + kWMaxStages;      // [kWDone] commit: unit u (mod kWDone) has been multiplied,
-                                                                  // its weight slots and activation stage are free
-    static constexpr int kBarDReady = kBarDone + kWDone;          // [kSets] commit: the chain is complete
-    static constexpr int kBarDFree = kBarDReady + kSets;          // [kSets] every decoder warp has read it
-    static constexpr int kBarCount = kBarDFree + kSets;
-    static_assert(kWDone >= kWMaxStages && kWDone >= 2 * kNA + 2, "a Done barrier must not be reused before it is waited for");
+    static constexpr int kBarCode = 0;                            // [kRing] TMA completion
+    static constexpr int kBarEmpty = kBarCode + kRing;            // [kRing] the eight warps that read the unit
+    static constexpr int kBarFull = kBarEmpty + kRing;            // [4] the group's four warps
+    static constexpr int kBarXFull = kBarFull + 4;                // [kWMaxStages] TMA completion
+    static constexpr int kBarDone = kBarXFull + kWMaxStages;      // [kWDone] both issuers' commits: half unit h (mod kWDone) has
+                                                                  // been multiplied, its weight slot and activation stage are free
+    static constexpr int kBarDReady = kBarDone + kWDone;          // [2 kSets] by MMA tile: its issuer's commit, the chain is complete
+    static constexpr int kBarDFree = kBarDReady + 2 * kSets;      // [2 kSets] the eight decoder warps that read it
+    static constexpr int kBarCount = kBarDFree + 2 * kSets;
+    static_assert(kWDone >= kWMaxStages && kWDone % 4 == 0, "a Done barrier must not be reused before it is waited for");
     static_assert(kBarCount * 8 + 64 <= kWBarBytes && kBarCount <= 96, "barrier block too small");
 };
 
@@ -173,15 +185,15 @@ struct WideWork {
 // Chains of one segment: its units cut into equal parts of at most kWChain.
 __device__ __forceinline__ int wide_chains(int units) { return (units + kWChain - 1) / kWChain; }
 
-template <int kCols, bool kFast>
-__global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constant__ WideArgs args) {
+template <int kCols, bool kFast, bool kConv>
+__global__ void __launch_bounds__(kConv ? kWConvThreads : kWThreads, 1) wide_kernel(const __grid_constant__ WideArgs args) {
     using Plan = WidePlan<kCols>;
-    constexpr int kNA = Plan::kNA, kSets = Plan::kSets;
+    constexpr int kThreads = kConv ? kWConvThreads : kWThreads;
+    constexpr int kSets = Plan::kSets, kRing = Plan::kRing;
     const WideParams &p = args.p;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t base = smem_u32(smem_raw);
     const uint32_t lut_addr = (base + kWPreBytes + 0xFFFFu) & ~0xFFFFu;
-    const uint32_t ring_addr = base + kWBarBytes;
     const uint32_t x_addr = lut_addr + kLutBytes;  // 1024-byte aligned, as the swizzle needs
     volatile int *flags = reinterpret_cast<volatile int *>(smem_raw + Plan::kBarCount * 8);  // [0]=failed [1]=last
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(smem_raw + Plan::kBarCount * 8 + 16);
@@ -189,7 +201,12 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint4 cb_pre = lut_prefetch(p.cb, tid);
-    if (x_addr + kWXBytes > base + p.dyn_smem_bytes) {  // uniform over the grid
+    // ring slots: kWRingPre below the table, the others behind the activation stages
+    auto ring_slot = [&](int rs) -> uint32_t {
+        return rs < kWRingPre ? base + kWBarBytes + static_cast<uint32_t>(rs) * kWUnitBytes
+                              : x_addr + Plan::kXBytes + static_cast<uint32_t>(rs - kWRingPre) * kWUnitBytes;
+    };
+    if (x_addr + kWPostBytes > base + p.dyn_smem_bytes) {  // uniform over the grid
         if (tid == 0) raise_status(DMM_STATUS_BAD_SMEM);
         return;
     }
@@ -202,14 +219,15 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
     bool bad_cb = false;
     if (warp < kWDecWarps) {
         bad_cb = lut_fill(lut_addr, p.cb, 1, p.sign_convention, kFmtHalf, tid, kWDecWarps * 32, true, &cb_pre);
-        named_barrier(4, kWThreads);
+        named_barrier(4, kThreads);
     } else {
         const int bt = tid - kWDecWarps * 32;
         if (bt < Plan::kBarCount) {
             uint32_t count = 1;                                                     // TMA completion, commit
             if (bt >= Plan::kBarEmpty && bt < Plan::kBarFull) count = 8;
             if (bt >= Plan::kBarFull && bt < Plan::kBarXFull) count = 4;
-            if (bt >= Plan::kBarDFree) count = kWDecWarps;
+            if (bt >= Plan::kBarDone && bt < Plan::kBarDReady) count = 2;
+            if (bt >= Plan::kBarDFree) count = kWDecWarps / 2;
             mbar_init(bar(bt), count);
             if (bt == 0) {
                 flags[0] = 0;
@@ -220,8 +238,8 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
         if (warp == kWMmaWarp) tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), kUTmemCols);
         fence_async_smem();
         tc_fence_before();
-        named_barrier(3, kWThreads - kWDecWarps * 32);
-        named_barrier_arrive(4, kWThreads);
+        named_barrier(3, kThreads - kWDecWarps * 32);
+        named_barrier_arrive(4, kThreads);
     }
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
@@ -237,96 +255,115 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
         if (bad_cb) raise_status(DMM_STATUS_BAD_CODEBOOK);
         const LutLane ll = lut_lane(lut_addr, lane, true);
         const uint32_t tlane = tmem + (static_cast<uint32_t>(wq * 32) << 16);
-        const uint32_t abase = tlane + Plan::kACol + static_cast<uint32_t>(q * kNA) * Plan::kSlotCols;
-        const int par = q >> 1, ki = q & 1;  // this group decodes k-tile ki of the units of parity par
-        const uint32_t lane_off = (wq * 4 + (lane >> 3)) * 256 + ki * 128 + (lane & 7) * 16;
-        const int mt = q >> 1;               // its part of the sums: MMA tile mt, column groups of parity q % 2
+        // this group decodes half `hf` of the units of parity `par`, into weight slot q
+        const int par = q >> 1, hf = q & 1;
+        const uint32_t acol = tlane + Plan::kACol + static_cast<uint32_t>(q) * Plan::kSlotCols;
+        const uint32_t lane_off = (wq * 4 + (lane >> 3)) * 512 + hf * 256 + (lane & 7) * 16;
+        const int mt = q >> 1;   // its part of the sums: MMA tile mt, column groups of parity q % 2
         int rs = par;            // ring slot of my next unit, and the parity of its barrier
         uint32_t cpar = 0;
-        int buf = 0;             // my next weight slot
+        constexpr int kFix = 3;  // partial tiles read at a time in the fix-up
         constexpr int kGroups = kCols / 32;  // groups of 16 columns whose sums this thread keeps
-        float sum[kGroups][16];
+        float sum[kGroups][16];  // of the chains of the current segment that have been read
+        auto clear_sums = [&] {
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g)
+#pragma unroll
+                for (int e = 0; e < 16; ++e) sum[g][e] = 0.f;
+        };
+        clear_sums();
 
         int un = 0;              // units of this CTA before the current chain
         int chains = 0;          // chains of this CTA so far (the accumulator set and the phase of its barriers)
-        WideSeg s = {}, prev = {};
-        bool pending = false, prev_first = false, prev_last = false;  // a chain that has not been read yet
-        for (int seg = 0, c = 0, nc = 0;;) {
+        bool code_ok = false;    // the codes of my next unit were seen to have landed
+        bool pending = false;    // there is a chain that has not been read yet
+        int ended = -1;          // the segment that it ends, if it does (looked up again then: registers are short here)
+        for (int seg = 0, c = 0, nc = 0, len = 0;;) {
             // next chain: c of nc of segment seg
             const bool more = seg < nseg;
             int u_end = un, first_part = un;
             if (more) {
                 if (c == 0) {
-                    s = work.get(seg);
-                    nc = wide_chains(s.u1 - s.u0);
+                    const WideSeg s = work.get(seg);
+                    len = s.u1 - s.u0;
+                    nc = wide_chains(len);
                 }
-                const int len = s.u1 - s.u0;
                 u_end = un + (len * (c + 1) / nc - len * c / nc);
-                // what is decoded before the previous chain is read: as many k-tiles as there are weight slots
-                first_part = pending ? (un + 2 * kNA < u_end ? un + 2 * kNA : u_end) : u_end;
+                // what is decoded before the previous chain is read: one half unit per group
+                first_part = pending ? (un + 2 < u_end ? un + 2 : u_end) : u_end;
             }
             int u = un + ((un ^ par) & 1);
             for (int part = 0; part < 2; ++part) {
                 const int stop = part == 0 ? first_part : u_end;
                 for (; u < stop; u += 2) {
-                    mbar_wait(bar(Plan::kBarCode + rs), cpar, flags);
-                    const uint32_t slot_addr = ring_addr + static_cast<uint32_t>(rs) * kWUnitBytes;
-                    uint4 cw;
-                    if constexpr (kFast)
-                        cw = fetch_fast_ktile(slot_addr, 2, wq, lane, ki);
-                    else
-                        cw = lds128(slot_addr + lane_off);
-                    const uint32_t w[4] = {cw.x, cw.y, cw.z, cw.w};
-                    // the slot held unit u - 2 kNA
-                    const int v = u - 2 * kNA;
-                    const uint32_t acol = abase + static_cast<uint32_t>(buf) * Plan::kSlotCols;
-                    uint32_t r[16];
-                    if constexpr (kCols <= 64) {
-                        uint32_t r1[16];
+                    if (!code_ok) mbar_wait(bar(Plan::kBarCode + rs), cpar, flags);
+                    const uint32_t slot_addr = ring_slot(rs);
+                    const int v = 2 * u + hf - 4;  // the half unit that the weight slot held before
+                    const bool done_ok = v < 0 || mbar_test(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1);
+                    uint4 cw[2];
 #pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            const uint4 d0 = decode8_half<0>(w[t], ll), d1 = decode8_half<1>(w[t], ll);
-                            r[4 * t] = d0.x; r[4 * t + 1] = d0.y; r[4 * t + 2] = d0.z; r[4 * t + 3] = d0.w;
-                            r1[4 * t] = d1.x; r1[4 * t + 1] = d1.y; r1[4 * t + 2] = d1.z; r1[4 * t + 3] = d1.w;
-                        }
-                        if (v >= 0) mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
-                        tc_fence_after();
-                        tmem_st16(acol, r);
-                        tmem_st16(acol + 16, r1);
-                    } else {  // one MMA tile after the other: the sums leave no registers for both
-#pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            const uint4 d = decode8_half<0>(w[t], ll);
-                            r[4 * t] = d.x; r[4 * t + 1] = d.y; r[4 * t + 2] = d.z; r[4 * t + 3] = d.w;
-                        }
-                        if (v >= 0) mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
-                        tc_fence_after();
-                        tmem_st16(acol, r);
-#pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            const uint4 d = decode8_half<1>(w[t], ll);
-                            r[4 * t] = d.x; r[4 * t + 1] = d.y; r[4 * t + 2] = d.z; r[4 * t + 3] = d.w;
-                        }
-                        tmem_st16(acol + 16, r);
+                    for (int i = 0; i < 2; ++i) {
+                        if constexpr (kFast)
+                            cw[i] = fetch_fast_ktile(slot_addr, 4, wq, lane, 2 * hf + i);
+                        else
+                            cw[i] = lds128(slot_addr + lane_off + i * 128);
                     }
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const uint32_t w[4] = {cw[i].x, cw[i].y, cw[i].z, cw[i].w};
+                        uint32_t r[16];
+                        if constexpr (kCols <= 64) {
+                            uint32_t r1[16];
+#pragma unroll
+                            for (int t = 0; t < 4; ++t) {
+                                const uint4 d0 = decode8_half<0>(w[t], ll), d1 = decode8_half<1>(w[t], ll);
+                                r[4 * t] = d0.x; r[4 * t + 1] = d0.y; r[4 * t + 2] = d0.z; r[4 * t + 3] = d0.w;
+                                r1[4 * t] = d1.x; r1[4 * t + 1] = d1.y; r1[4 * t + 2] = d1.z; r1[4 * t + 3] = d1.w;
+                            }
+                            if (i == 0) {
+                                if (!done_ok) mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
+                                tc_fence_after();
+                            }
+                            tmem_st16(acol + i * 32, r);
+                            tmem_st16(acol + i * 32 + 16, r1);
+                        } else {  // one MMA tile after the other: the sums leave no registers for both
+#pragma unroll
+                            for (int t = 0; t < 4; ++t) {
+                                const uint4 d = decode8_half<0>(w[t], ll);
+                                r[4 * t] = d.x; r[4 * t + 1] = d.y; r[4 * t + 2] = d.z; r[4 * t + 3] = d.w;
+                            }
+                            if (i == 0) {
+                                if (!done_ok) mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
+                                tc_fence_after();
+                            }
+                            tmem_st16(acol + i * 32, r);
+#pragma unroll
+                            for (int t = 0; t < 4; ++t) {
+                                const uint4 d = decode8_half<1>(w[t], ll);
+                                r[4 * t] = d.x; r[4 * t + 1] = d.y; r[4 * t + 2] = d.z; r[4 * t + 3] = d.w;
+                            }
+                            tmem_st16(acol + i * 32 + 16, r);
+                        }
+                    }
+                    const int rs_done = rs;
+                    rs += 2;
+                    if (rs >= kRing) {
+                        rs -= kRing;
+                        cpar ^= 1u;
+                    }
+                    code_ok = mbar_test(bar(Plan::kBarCode + rs), cpar);
                     tmem_wait_st();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
-                        mbar_arrive(bar(Plan::kBarFull + q * kNA + buf));
-                        mbar_arrive(bar(Plan::kBarEmpty + rs));
-                    }
-                    if (++buf == kNA) buf = 0;
-                    rs += 2;
-                    if (rs >= kWRing) {
-                        rs -= kWRing;
-                        cpar ^= 1u;
+                        mbar_arrive(bar(Plan::kBarFull + q));
+                        mbar_arrive(bar(Plan::kBarEmpty + rs_done));
                     }
                 }
                 if (part == 0 && pending) {
                     // ---------------- the previous chain: its accumulators into the sums ----------------
                     const int set = (chains - 1) & (kSets - 1);
-                    mbar_wait(bar(Plan::kBarDReady + set), ((chains - 1) / kSets) & 1, flags);
+                    mbar_wait(bar(Plan::kBarDReady + 2 * set + mt), ((chains - 1) / kSets) & 1, flags);
                     tc_fence_after();
                     const uint32_t dcol = tlane + static_cast<uint32_t>(set) * Plan::kSetCols + static_cast<uint32_t>(mt * kCols);
 #pragma unroll
@@ -338,16 +375,16 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
                             tmem_ld16(dcol + static_cast<uint32_t>(b0), a);
                             tmem_wait_ld(a);
 #pragma unroll
-                            for (int e = 0; e < 16; ++e)
-                                sum[g][e] = prev_first ? __uint_as_float(a[e]) : sum[g][e] + __uint_as_float(a[e]);
+                            for (int e = 0; e < 16; ++e) sum[g][e] += __uint_as_float(a[e]);
                         }
                     }
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(Plan::kBarDFree + set));
+                    if (lane == 0) mbar_arrive(bar(Plan::kBarDFree + 2 * set + mt));
 
-                    if (prev_last) {
+                    if (ended >= 0) {
                         // ---------------- epilogue of the previous segment ----------------
+                        const WideSeg prev = work.get(ended);
                         const int trow = wq * 32 + lane;
                         const long long n = kFast ? static_cast<long long>(prev.ss) * 256 + 32 * (4 * mt + wq) + lane
                                                   : (static_cast<long long>(prev.ss) * 16 + wq * 4 + (lane >> 3)) * 16 + 8 * mt + (lane & 7);
@@ -408,14 +445,22 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
                                         float v[16];
 #pragma unroll
                                         for (int e = 0; e < 16; ++e) v[e] = 0.f;
-                                        for (int cc = c_lo; cc <= c_hi; ++cc) {  // fixed summation order, sixteen loads in flight
-                                            const float *src = p.partials + (2ll * cc + (part32_begin(p.part, cc) > a ? 0 : 1)) * part_sz +
-                                                               (static_cast<long long>(mt) * p.nb + b0) * 128 + trow;
-                                            float l[16];
+                                        // fixed summation order; kFix contributors at a time
+                                        for (int c0 = c_lo; c0 <= c_hi; c0 += kFix) {
+                                            float l[kFix][16];
 #pragma unroll
-                                            for (int e = 0; e < 16; ++e) l[e] = b0 + e < mcols ? __ldcg(src + e * 128) : 0.f;
+                                            for (int k = 0; k < kFix; ++k) {
+                                                const int cc = c0 + k <= c_hi ? c0 + k : c_hi;
+                                                const float *src = p.partials + (2ll * cc + (part32_begin(p.part, cc) > a ? 0 : 1)) * part_sz +
+                                                                   (static_cast<long long>(mt) * p.nb + b0) * 128 + trow;
 #pragma unroll
-                                            for (int e = 0; e < 16; ++e) v[e] += l[e];
+                                                for (int e = 0; e < 16; ++e)
+                                                    l[k][e] = b0 + e < mcols && c0 + k <= c_hi ? __ldcg(src + e * 128) : 0.f;
+                                            }
+#pragma unroll
+                                            for (int k = 0; k < kFix; ++k)
+#pragma unroll
+                                                for (int e = 0; e < 16; ++e) v[e] += l[k][e];
                                         }
                                         if (row_ok) {
 #pragma unroll
@@ -427,6 +472,7 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
                             }
                             named_barrier(1, kWDecWarps * 32);  // flags[1] is reused by the next segment
                         }
+                        clear_sums();
                     }
                 }
             }
@@ -434,65 +480,63 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
             un = u_end;
             ++chains;
             pending = true;
-            prev = s;
-            prev_first = c == 0;
-            prev_last = c + 1 == nc;
+            ended = -1;
             if (++c == nc) {
                 c = 0;
-                ++seg;
+                ended = seg++;
             }
         }
-    } else if (warp == kWMmaWarp) {
-        // =============================== MMA issuer ===============================
+    } else if (warp < kWCodeWarp) {
+        // =============================== MMA issuers ===============================
+        const int mt = warp - kWMmaWarp;
         const bool leader = elect_one();
         // D fp32 (1 at bit 4), A and B fp16 (0), N >> 3 at bit 17, M >> 4 at bit 24
         const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(p.nb >> 3) << 17) | ((128u >> 4) << 24);
         // 128-byte swizzle (2 at bit 61), 8-row groups 1024 bytes apart, version 1 at bit 46
         const uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-        const uint32_t a0 = tmem + Plan::kACol;
+        const uint32_t a0 = tmem + Plan::kACol + static_cast<uint32_t>(mt * 16);
+        const uint32_t d0 = tmem + static_cast<uint32_t>(mt * kCols);
         const uint32_t x16 = ((x_addr >> 4) & 0x3FFFu) | (1u << 16), stage16 = stage_b >> 4;
-        int xs = 0, buf = 0, un = 0, chains = 0;
-        uint32_t xpar = 0, fullpar = 0;
+        int xs = 0, h = 0, chains = 0;  // h: half units of this CTA so far
+        uint32_t xpar = 0;
+        bool x_ok = false, a_ok = false;  // the operands of the next half unit were seen to be ready
         for (int seg = 0; seg < nseg; ++seg) {
             const WideSeg s = work.get(seg);
             const int len = s.u1 - s.u0, nc = wide_chains(len);
             for (int c = 0; c < nc; ++c, ++chains) {
                 const int set = chains & (kSets - 1);
                 if (chains >= kSets) {
-                    mbar_wait(bar(Plan::kBarDFree + set), ((chains / kSets) - 1) & 1, flags);
+                    mbar_wait(bar(Plan::kBarDFree + 2 * set + mt), ((chains / kSets) - 1) & 1, flags);
                     tc_fence_after();
                 }
-                const uint32_t d = tmem + static_cast<uint32_t>(set) * Plan::kSetCols;
+                const uint32_t d = d0 + static_cast<uint32_t>(set) * Plan::kSetCols;
                 uint32_t acc = 0u;
                 const int n = len * (c + 1) / nc - len * c / nc;
-                for (int u = 0; u < n; ++u, ++un) {
-                    mbar_wait(bar(Plan::kBarXFull + xs), xpar, flags);
+                for (int e = 0; e < 2 * n; ++e) {
+                    const int sl = h & 3;
+                    if (!x_ok) mbar_wait(bar(Plan::kBarXFull + xs), xpar, flags);
+                    if (!a_ok) mbar_wait(bar(Plan::kBarFull + sl), (h >> 2) & 1, flags);
+                    tc_fence_after();
                     const uint32_t xlo = x16 + static_cast<uint32_t>(xs) * stage16;
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const int sl = ((un & 1) * 2 + i) * kNA + buf;  // the unit's parity and k-tile name the decoder group
-                        mbar_wait(bar(Plan::kBarFull + sl), fullpar, flags);
-                        tc_fence_after();
-                        if (leader) {
-                            const uint32_t a = a0 + static_cast<uint32_t>(sl) * Plan::kSlotCols;
-                            mma_ts_f16_lh(d, a, xlo + i * 4, desc_hi, idesc, acc);
-                            mma_ts_f16_lh(d + kCols, a + 16, xlo + i * 4, desc_hi, idesc, acc);
-                            mma_ts_f16_lh(d, a + 8, xlo + i * 4 + 2, desc_hi, idesc, 1u);
-                            mma_ts_f16_lh(d + kCols, a + 24, xlo + i * 4 + 2, desc_hi, idesc, 1u);
-                        }
-                        acc = 1u;
-                    }
-                    if (leader) tc_commit(bar(Plan::kBarDone + (un & (kWDone - 1))));
+                    const uint32_t a = a0 + static_cast<uint32_t>(sl) * Plan::kSlotCols;
+                    const int done = h & (kWDone - 1);
+                    ++h;
                     if (++xs == p.stages) {
                         xs = 0;
                         xpar ^= 1u;
                     }
-                    if ((un & 1) != 0 && ++buf == kNA) {
-                        buf = 0;
-                        fullpar ^= 1u;
+                    x_ok = mbar_test(bar(Plan::kBarXFull + xs), xpar);
+                    a_ok = mbar_test(bar(Plan::kBarFull + (h & 3)), (h >> 2) & 1);
+                    if (leader) {
+                        mma_ts_f16_lh(d, a, xlo, desc_hi, idesc, acc);
+                        mma_ts_f16_lh(d, a + 8, xlo + 2, desc_hi, idesc, 1u);
+                        mma_ts_f16_lh(d, a + 32, xlo + 4, desc_hi, idesc, 1u);
+                        mma_ts_f16_lh(d, a + 40, xlo + 6, desc_hi, idesc, 1u);
+                        tc_commit(bar(Plan::kBarDone + done));
                     }
+                    acc = 1u;
                 }
-                if (leader) tc_commit(bar(Plan::kBarDReady + set));
+                if (leader) tc_commit(bar(Plan::kBarDReady + 2 * set + mt));
             }
         }
     } else if (warp == kWCodeWarp) {
@@ -506,23 +550,79 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
             for (int seg = 0; seg < nseg; ++seg) {
                 const WideSeg s = work.get(seg);
                 for (int u = s.u0; u < s.u1; ++u, ++n) {
-                    if (n >= kWRing) mbar_wait(bar(Plan::kBarEmpty + rs), par, flags);
+                    if (n >= kRing) mbar_wait(bar(Plan::kBarEmpty + rs), par, flags);
                     const uint32_t b = bar(Plan::kBarCode + rs);
                     mbar_arrive_expect_tx(b, kWUnitBytes);
                     // always the full box: words past the row or strips past N read as zero
-                    tma_load_2d(ring_addr + static_cast<uint32_t>(rs) * kWUnitBytes, &args.codes_map, kFast ? u * 128 : u * 64,
+                    tma_load_2d(ring_slot(rs), &args.codes_map, kFast ? u * 256 : u * 128,
                                 kFast ? s.ss * 8 : s.ss * 16, b, policy);
-                    if (++rs == kWRing) {
+                    if (++rs == kRing) {
                         rs = 0;
                         par ^= 1u;
                     }
                 }
             }
             if (flags[0]) {  // a wait gave up: let the loads in flight land before the CTA exits
-                for (uint32_t e = 0; e < kWRing && e < n; ++e) {
+                for (uint32_t e = 0; e < kRing && e < n; ++e) {
                     const uint32_t i = n - 1 - e;
-                    mbar_wait_limit(bar(Plan::kBarCode + static_cast<int>(i % kWRing)), (i / kWRing) & 1, 20ll * 1000 * 1000);
+                    mbar_wait_limit(bar(Plan::kBarCode + static_cast<int>(i % kRing)), (i / kRing) & 1, 20ll * 1000 * 1000);
                 }
+            }
+        }
+    } else if (kConv) {
+        // ======================= activation loaders: fp32 to fp16 =======================
+        grid_dep_wait();
+        if (warp == kWClearWarp) {
+            if (p.zero_ptr != nullptr)  // a later kernel will accumulate into it
+                for (long long i = static_cast<long long>(blockIdx.x) * 32 + lane; i < p.zero_count;
+                     i += static_cast<long long>(gridDim.x) * 32)
+                    p.zero_ptr[i] = 0.f;
+        } else {
+            const int total = static_cast<int>(p.M) * 8;  // pieces of a unit: 8 k of one row, 16 bytes of shared memory
+            const int ns = p.stages;
+            int n = warp - kWXWarp, nbase = 0;
+            for (int seg = 0; seg < nseg; ++seg) {
+                const WideSeg s = work.get(seg);
+                const int nend = nbase + 2 * (s.u1 - s.u0);  // half units
+                for (; n < nend; n += kWLoaders) {
+                    const int k0 = (2 * s.u0 + n - nbase) * 64, xs = n % ns;
+                    const uint32_t stage = x_addr + static_cast<uint32_t>(xs) * stage_b;
+                    for (int p0 = 0; p0 < total; p0 += 128) {
+                        // All loads of the four pieces first, at addresses that are always valid: with a branch around
+                        // each piece they went out one after the other.  (Rows past M are not written: they only
+                        // reach accumulator columns that nobody reads.  k past the row is zero.)
+                        float4 f[4][2], g[4][2];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int pc = min(p0 + e * 32 + lane, total - 1), k = k0 + (pc & 7) * 8;
+                            const float *src = reinterpret_cast<const float *>(p.x) + (pc >> 3) * p.x_ld + (k < p.K ? k : 0);
+                            f[e][0] = __ldcg(reinterpret_cast<const float4 *>(src));
+                            f[e][1] = __ldcg(reinterpret_cast<const float4 *>(src + 4));
+                            if (p.x_mode == kXSiluMul) {
+                                g[e][0] = __ldcg(reinterpret_cast<const float4 *>(src + p.x_gap));
+                                g[e][1] = __ldcg(reinterpret_cast<const float4 *>(src + p.x_gap + 4));
+                            }
+                        }
+                        if (p0 == 0 && n >= ns) {  // the stage held half unit n - ns
+                            const int v = n - ns;
+                            mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int pc = p0 + e * 32 + lane, row = pc >> 3, ch = pc & 7;
+                            uint32_t h[4];
+                            pack_piece(p.x_mode, f[e], g[e], h);
+                            const bool in = k0 + ch * 8 < p.K;
+                            if (pc < total)
+                                sts128(stage + row * 128 + ((ch ^ (row & 7)) << 4),
+                                       make_uint4(in ? h[0] : 0u, in ? h[1] : 0u, in ? h[2] : 0u, in ? h[3] : 0u));
+                        }
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(Plan::kBarXFull + xs));
+                }
+                nbase = nend;
             }
         }
     } else if (warp == kWXWarp) {
@@ -535,8 +635,8 @@ __global__ void __launch_bounds__(kWThreads, 1) wide_kernel(const __grid_constan
             const uint32_t ns = static_cast<uint32_t>(p.stages);
             for (int seg = 0; seg < nseg; ++seg) {
                 const WideSeg s = work.get(seg);
-                for (int u = s.u0; u < s.u1; ++u, ++n) {
-                    if (n >= ns) {  // the stage held unit n - ns
+                for (int u = 2 * s.u0; u < 2 * s.u1; ++u, ++n) {
+                    if (n >= ns) {  // the stage held half unit n - ns
                         const uint32_t v = n - ns;
                         mbar_wait(bar(Plan::kBarDone + static_cast<int>(v & (kWDone - 1))), (v / kWDone) & 1, flags);
                     }
@@ -619,9 +719,9 @@ inline int make_x_map(CUtensorMap *map, const void *x, long long M, long long K,
     return r == CUDA_SUCCESS ? 0 : static_cast<int>(cudaErrorInvalidValue);
 }
 
-template <int kCols, bool kFast>
+template <int kCols, bool kFast, bool kConv>
 inline int launch_wide_as(WideArgs &args, unsigned grid, bool pdl, cudaStream_t stream) {
-    auto kernel = wide_kernel<kCols, kFast>;
+    auto kernel = wide_kernel<kCols, kFast, kConv>;
     // the shared-memory attribute is set once per kernel variant and device, not on every launch
     static std::atomic<unsigned long long> attr_done;
     int dev = 0;
@@ -634,7 +734,7 @@ inline int launch_wide_as(WideArgs &args, unsigned grid, bool pdl, cudaStream_t 
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kWThreads);
+    cfg.blockDim = dim3(kConv ? kWConvThreads : kWThreads);
     cfg.dynamicSmemBytes = kWDynBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -646,12 +746,12 @@ inline int launch_wide_as(WideArgs &args, unsigned grid, bool pdl, cudaStream_t 
 }
 
 // p carries cb, out, partials, tickets, M, N, scale, flags, sign convention and the buffer to clear; x is fp16
-// [M, K] with rows x_ld elements apart.  partial_capacity: bytes of workspace behind p.partials; n_tickets: counters at p.tickets.
-inline int launch_wide(WideParams p, const void *x, long long x_ld, const void *codes, long long K, bool fast_layout,
+// [M, K] with rows x_ld elements apart, or fp32 as x_mode says (at most kWConvRows rows).  partial_capacity: bytes of workspace behind p.partials; n_tickets: counters at p.tickets.
+inline int launch_wide(WideParams p, const void *x, int x_mode, long long x_ld, long long x_gap, const void *codes, long long K, bool fast_layout,
                        size_t partial_capacity, long long n_tickets, int num_sms, bool pdl, cudaStream_t stream) {
     WideArgs args = {};
     p.nb = wide_cols(p.M);
-    p.units = static_cast<int>((K + 63) / 64);
+    p.units = static_cast<int>((K + 127) / 128);
     p.sst = static_cast<int>((p.N + 255) / 256);
     const long long tiles = static_cast<long long>(p.sst) * ((p.M + p.nb - 1) / p.nb);
     if (tiles * p.units >= (1ll << 31)) return DMM_ERR_SHAPE;
@@ -659,10 +759,19 @@ inline int launch_wide(WideParams p, const void *x, long long x_ld, const void *
     long long grid = whole > 0 ? num_sms : 0;
     const bool can_split = p.atomic_reduce || (partial_capacity >= wide_partial_bytes(p.M, num_sms) && rest <= n_tickets);
     if (rest > 0) {
-        // at least two units per CTA: below that the pipeline's fill costs more than the split gains
-        long long parts = can_split ? rest * p.units / 2 : rest;
-        if (parts < rest) parts = rest;
-        if (parts > num_sms) parts = num_sms;
+        // How many CTAs share the remaining tiles: estimated cycles of the longest CTA.  A unit costs about
+        // 640 + 10 nb, and a split tile a fix-up: its last CTA reads nb KiB per contributor at 64 bytes a cycle.
+        long long parts = rest, best = 0;
+        for (long long c = rest; can_split && c <= num_sms; c = c < num_sms && c + rest > num_sms ? num_sms : c + rest) {
+            if (c > rest && c > rest * p.units) break;
+            const long long n = (rest * p.units + c - 1) / c, contributors = c == rest ? 0 : (c + rest - 1) / rest + 1;
+            const long long fix = contributors == 0 ? 0 : 3000 + 16 * p.nb * (p.atomic_reduce ? 1 : contributors + 1);
+            const long long cost = n * (640 + 10 * p.nb) + fix;
+            if (best == 0 || cost < best) {
+                best = cost;
+                parts = c;
+            }
+        }
         p.split_grid = static_cast<int>(parts);
         if (!can_split) {  // one whole tile each
             p.part.a = p.units;
@@ -674,18 +783,34 @@ inline int launch_wide(WideParams p, const void *x, long long x_ld, const void *
         if (parts > grid) grid = parts;
     }
     p.whole = static_cast<int>(whole);
-    const int fit = static_cast<int>(kWXBytes / (static_cast<uint32_t>(p.nb) * 128u));
+    const uint32_t x_bytes = p.nb <= 32 ? WidePlan<32>::kXBytes : (p.nb <= 64 ? WidePlan<64>::kXBytes : WidePlan<128>::kXBytes);
+    const int fit = static_cast<int>(x_bytes / (static_cast<uint32_t>(p.nb) * 128u));
     p.stages = fit < kWMaxStages ? fit : kWMaxStages;
     p.dyn_smem_bytes = kWDynBytes;
+    p.x = x;
+    p.x_mode = x_mode;
+    p.x_ld = x_ld;
+    p.x_gap = x_gap;
+    p.K = K;
     args.p = p;
-    int rc = make_codes_map(&args.codes_map, codes, p.N, K, 2, fast_layout);
-    if (rc) return rc;
-    rc = make_x_map(&args.x_map, x, p.M, K, x_ld, p.nb);
+    int rc = make_codes_map(&args.codes_map, codes, p.N, K, 4, fast_layout);
     if (rc) return rc;
     const unsigned g = static_cast<unsigned>(grid);
-    if (p.nb <= 32) return fast_layout ? launch_wide_as<32, true>(args, g, pdl, stream) : launch_wide_as<32, false>(args, g, pdl, stream);
-    if (p.nb <= 64) return fast_layout ? launch_wide_as<64, true>(args, g, pdl, stream) : launch_wide_as<64, false>(args, g, pdl, stream);
-    return fast_layout ? launch_wide_as<128, true>(args, g, pdl, stream) : launch_wide_as<128, false>(args, g, pdl, stream);
+    if (x_mode != kXHalf) {
+        if (p.M > kWConvRows) return DMM_ERR_SHAPE;
+        return fast_layout ? launch_wide_as<32, true, true>(args, g, pdl, stream)
+                           : launch_wide_as<32, false, true>(args, g, pdl, stream);
+    }
+    rc = make_x_map(&args.x_map, x, p.M, K, x_ld, p.nb);
+    if (rc) return rc;
+    if (p.nb <= 32)
+        return fast_layout ? launch_wide_as<32, true, false>(args, g, pdl, stream)
+                           : launch_wide_as<32, false, false>(args, g, pdl, stream);
+    if (p.nb <= 64)
+        return fast_layout ? launch_wide_as<64, true, false>(args, g, pdl, stream)
+                           : launch_wide_as<64, false, false>(args, g, pdl, stream);
+    return fast_layout ? launch_wide_as<128, true, false>(args, g, pdl, stream)
+                       : launch_wide_as<128, false, false>(args, g, pdl, stream);
 }
 
 }  // namespace dmm
