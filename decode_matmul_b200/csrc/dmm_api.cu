@@ -75,7 +75,19 @@ static size_t partial_bytes(long long M, int num_sms) {
 static size_t planes_offset(long long M, long long N, int num_sms) {
     return (ticket_bytes(N) + partial_bytes(M, num_sms) + 255) & ~static_cast<size_t>(255);
 }
-constexpr long long kWideMinBatch = 17;  // from this batch on the wide kernel runs
+// Which kernel a product of the fp16 family runs on: the wide one (dmm_wide.cuh) or the fp8-plane kernels.  Per
+// tile of codes (256 rows x 32 k) and SM the wide kernel costs more up to some 32 rows, per call it costs less (no
+// planes kernel, a cheaper fix-up), so the line is a number of tiles per SM.  Microseconds, planes / wide:
+//   fp16 in, own result   4 x 4096 x 4096 13.5 / 8.8, 4 x 28672 x 8192 26.6 / 34.6; 8 x 8192 x 8192 17.6 / 17.3, 8 x
+//                         57344 x 8192 45 / 62; 16 x 28672 x 8192 35.7 / 35.4, 16 x 57344 x 8192 55 / 62; from 17
+//                         rows on always (32 x 28672 x 8192 48 / 36)
+//   added into a stack    a block of the 7B model at 16 rows 57.8 / 51.7, at 24 69.9 / 60.7; of the 70B model at 16
+//                         112 / 148, at 24 137 / 147; from 33 rows on the planes take two passes
+static bool wide_is_faster(long long M, long long N, long long K, bool fused, int num_sms) {
+    const long long per_sm = (N + 255) / 256 * (K / 32) / num_sms;
+    if (fused) return M > 32 || (M > 16 ? per_sm <= 107 : M > 8 && per_sm <= 60);
+    return M > 16 || (M >= 4 && per_sm <= 15 * M - 28);
+}
 
 static size_t workspace_need(long long M, long long N, long long K, int num_sms) {
     return planes_offset(M, N, num_sms) + static_cast<size_t>(K) * 128;
@@ -269,14 +281,15 @@ struct TpArgs {
 static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long long x_gap, const void *codes,
                     const void *cb16, float scale, float *out, long long M, long long N, long long K,
                     int sign_convention, unsigned flags, void *workspace, size_t workspace_bytes, cudaStream_t stream,
-                    float *zero_ptr = nullptr, long long zero_count = 0, const TpArgs *tp = nullptr, bool fast_layout = false) {
+                    float *zero_ptr = nullptr, long long zero_count = 0, const TpArgs *tp = nullptr, bool fast_layout = false,
+                    bool may_go_wide = false) {
     DeviceState *d = nullptr;
     int rc = current_device_state(&d);
     if (rc) return rc;
     void *ws = nullptr;
     rc = resolve_workspace(d, M, N, K, workspace, workspace_bytes, stream, &ws);
     if (rc) return rc;
-    if (f8 && M >= kWideMinBatch && tp == nullptr)
+    if (may_go_wide && wide_is_faster(M, N, K, x_kind != DMM_X_F16 || (flags & DMM_FLAG_ATOMIC) != 0, d->num_sms))
         return run_wide(x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K, sign_convention, flags, workspace,
                         workspace_bytes, stream, zero_ptr, zero_count, fast_layout);
     const long long step = f8 ? 32 : 64;
@@ -449,7 +462,8 @@ int dmm_f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, const 
     if (x_ld < K || x_ld % 8 != 0 || x_gap % 4 != 0 || (x_kind == DMM_X_F32_SILU_MUL && x_gap + K > x_ld))
         return DMM_ERR_SHAPE;
     if (zero_count < 0 || (zero_count > 0 && zero_ptr == nullptr)) return DMM_ERR_ARG;
-    if (path == DMM_PATH_AUTO) path = x_kind == DMM_X_F16 ? dmm_select_path(M, N, K) : DMM_PATH_TCGEN05_F8;
+    const bool any_path = path == DMM_PATH_AUTO;
+    if (any_path) path = x_kind == DMM_X_F16 ? dmm_select_path(M, N, K) : DMM_PATH_TCGEN05_F8;
     bool fast_native = false;
     if (layout == DMM_LAYOUT_FAST) {
         if (N % 32 != 0) return DMM_ERR_SHAPE;
@@ -471,7 +485,7 @@ int dmm_f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, const 
     if (path == DMM_PATH_TCGEN05 || path == DMM_PATH_TCGEN05_F8)
         return run_umma(path == DMM_PATH_TCGEN05_F8, x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K,
                         sign_convention, flags, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), zero_ptr,
-                        zero_count, nullptr, fast_native);
+                        zero_count, nullptr, fast_native, any_path && path == DMM_PATH_TCGEN05_F8);
     if (x_ld != K) return DMM_ERR_UNSUPPORTED;
     // the streaming kernel accumulates quarter units: fold the 1/4 into the scale
     return run_stream(1, x, codes, cb16, 1, 0.25f * scale, out, M, N, K, sign_convention, flags, workspace,
@@ -811,7 +825,7 @@ size_t dmm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
     int sms = 256;
     if (current_device_state(&d) == 0 && d->num_sms > 0) sms = d->num_sms;
     size_t need = workspace_need(M, N, K, sms);
-    if (M >= kWideMinBatch) {  // (with less the wide kernel leaves the last tiles whole)
+    if (M > 64) {  // (with less the wide kernel leaves the last tiles whole)
         const size_t wide = ticket_bytes(N) + wide_partial_bytes(M, sms);
         if (wide > need) need = wide;
     }
@@ -863,8 +877,8 @@ int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_con
 }
 
 int dmm_select_path(int64_t M, int64_t N, int64_t K) {
-    // Measured on B200: the fp6/fp8-operand kernel (32 batch rows per pass, planes split once by
-    // planes_kernel from 4 rows on) beats the fp16-operand one at every batch size.
+    // Measured on B200: fp6 weights and fp8 activation planes beat the fp16-operand policy of the same kernel at every
+    // batch size.  On DMM_PATH_AUTO the wide fp16-operand kernel takes over where it is faster (wide_is_faster).
     (void)M;
     (void)N;
     (void)K;

@@ -43,7 +43,7 @@
 //          warp 16 allocates the tensor memory
 //   18     TMA producer of the codes (one thread), 19 of the activations (the only thread whose loads
 //          depend on the previous kernel of the stream); warp 19 also clears zero_ptr.
-//   kConv (fp32 activations, plain or silu(gate) * up, up to 32 batch rows): warps 19..22 load the activations
+//   kConv (fp32 activations, plain or silu(gate) * up, up to 16 batch rows): warps 19..22 load the activations
 //          of every fourth half unit each, round them to fp16 and store them as the TMA would have; warp 23 clears
 //          zero_ptr.  A kernel that converts them beforehand costs a launch per product, more than this.
 // Every wait is bounded (mbar_wait).
@@ -55,7 +55,8 @@ namespace dmm {
 constexpr int kWDecWarps = 16, kWMmaWarp = 16, kWCodeWarp = 18, kWXWarp = 19;
 constexpr int kWThreads = 20 * 32;
 constexpr int kWConvThreads = 24 * 32, kWLoaders = 4, kWClearWarp = 23;
-constexpr int kWConvRows = 32;                  // batch rows up to which the kernel converts fp32 activations itself
+constexpr int kWConvRows = 16;                  // batch rows up to which the kernel converts fp32 activations itself
+                                                // (one piece per lane and quarter; with 32 rows the loaders fall behind)
 constexpr int kWMaxCols = 128;
 constexpr int kWChain = 11;                     // units (of eight MMAs per accumulator) before the sums leave the tensor core
 constexpr int kWDone = 16;                      // ring of "half unit done" barriers
@@ -587,36 +588,34 @@ __global__ void __launch_bounds__(kConv ? kWConvThreads : kWThreads, 1) wide_ker
                 for (; n < nend; n += kWLoaders) {
                     const int k0 = (2 * s.u0 + n - nbase) * 64, xs = n % ns;
                     const uint32_t stage = x_addr + static_cast<uint32_t>(xs) * stage_b;
-                    for (int p0 = 0; p0 < total; p0 += 128) {
-                        // All loads of the four pieces first, at addresses that are always valid: with a branch around
-                        // each piece they went out one after the other.  (Rows past M are not written: they only
-                        // reach accumulator columns that nobody reads.  k past the row is zero.)
-                        float4 f[4][2], g[4][2];
+                    // All loads of the four pieces first, at addresses that are always valid: with a branch around
+                    // each piece they went out one after the other.  (Rows past M are not written: they only
+                    // reach accumulator columns that nobody reads.  k past the row is zero.)
+                    float4 f[4][2], g[4][2];
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int pc = min(p0 + e * 32 + lane, total - 1), k = k0 + (pc & 7) * 8;
-                            const float *src = reinterpret_cast<const float *>(p.x) + (pc >> 3) * p.x_ld + (k < p.K ? k : 0);
-                            f[e][0] = __ldcg(reinterpret_cast<const float4 *>(src));
-                            f[e][1] = __ldcg(reinterpret_cast<const float4 *>(src + 4));
-                            if (p.x_mode == kXSiluMul) {
-                                g[e][0] = __ldcg(reinterpret_cast<const float4 *>(src + p.x_gap));
-                                g[e][1] = __ldcg(reinterpret_cast<const float4 *>(src + p.x_gap + 4));
-                            }
+                    for (int e = 0; e < 4; ++e) {
+                        const int pc = min(e * 32 + lane, total - 1), k = k0 + (pc & 7) * 8;
+                        const float *src = reinterpret_cast<const float *>(p.x) + (pc >> 3) * p.x_ld + (k < p.K ? k : 0);
+                        f[e][0] = __ldcg(reinterpret_cast<const float4 *>(src));
+                        f[e][1] = __ldcg(reinterpret_cast<const float4 *>(src + 4));
+                        if (p.x_mode == kXSiluMul) {
+                            g[e][0] = __ldcg(reinterpret_cast<const float4 *>(src + p.x_gap));
+                            g[e][1] = __ldcg(reinterpret_cast<const float4 *>(src + p.x_gap + 4));
                         }
-                        if (p0 == 0 && n >= ns) {  // the stage held half unit n - ns
-                            const int v = n - ns;
-                            mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
-                        }
+                    }
+                    if (n >= ns) {  // the stage held half unit n - ns
+                        const int v = n - ns;
+                        mbar_wait(bar(Plan::kBarDone + (v & (kWDone - 1))), (v / kWDone) & 1, flags);
+                    }
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int pc = p0 + e * 32 + lane, row = pc >> 3, ch = pc & 7;
-                            uint32_t h[4];
-                            pack_piece(p.x_mode, f[e], g[e], h);
-                            const bool in = k0 + ch * 8 < p.K;
-                            if (pc < total)
-                                sts128(stage + row * 128 + ((ch ^ (row & 7)) << 4),
-                                       make_uint4(in ? h[0] : 0u, in ? h[1] : 0u, in ? h[2] : 0u, in ? h[3] : 0u));
-                        }
+                    for (int e = 0; e < 4; ++e) {
+                        const int pc = e * 32 + lane, row = pc >> 3, ch = pc & 7;
+                        uint32_t h[4];
+                        pack_piece(p.x_mode, f[e], g[e], h);
+                        const bool in = k0 + ch * 8 < p.K;
+                        if (pc < total)
+                            sts128(stage + row * 128 + ((ch ^ (row & 7)) << 4),
+                                   make_uint4(in ? h[0] : 0u, in ? h[1] : 0u, in ? h[2] : 0u, in ? h[3] : 0u));
                     }
                     fence_async_smem();
                     __syncwarp();

@@ -1,4 +1,4 @@
-"""The wide fp16-operand kernel (17 batch rows and more) against the CPU oracle, at the sizes where its tiles,
+"""The wide fp16-operand kernel (larger batches, and smaller ones on small matrices) against the CPU oracle, at the sizes where its tiles,
 units and splits end.  Needs a B200."""
 import numpy as np
 import pytest
@@ -45,7 +45,7 @@ def _rel(y, want):
 
 
 # rows around every column-tile size (64, 128, 192 and their multiples), N around 256, K around 64 and 128
-SHAPES = [(17, 16, 32), (17, 272, 64), (31, 256, 96), (32, 528, 1056), (33, 240, 2048), (48, 4096, 544), (64, 512, 512),
+SHAPES = [(4, 16, 32), (5, 528, 1056), (16, 512, 160), (17, 16, 32), (17, 272, 64), (31, 256, 96), (32, 528, 1056), (33, 240, 2048), (48, 4096, 544), (64, 512, 512),
           (65, 512, 160), (128, 272, 1024), (129, 256, 2048), (192, 320, 128), (193, 528, 1056), (333, 1024, 512),
           (400, 16, 96), (577, 4096, 128), (1000, 9472, 64)]
 
@@ -83,7 +83,7 @@ def test_accumulate_and_scale(M, atomic):
     assert _rel(y.cpu().numpy(), base + 0.125 * _want(x, codes, cb16)) <= REL
 
 
-@pytest.mark.parametrize("M", [17, 64, 65, 150])
+@pytest.mark.parametrize("M", [9, 16, 17, 64, 65, 150])
 @pytest.mark.parametrize("silu", [False, True])
 def test_fp32_inputs_and_clearing(M, silu):
     """fp32 activations are rounded to fp16 first, as the narrower kernels do; `zero` is cleared on the way."""
@@ -101,6 +101,41 @@ def test_fp32_inputs_and_clearing(M, silu):
     # silu in the kernel uses the fast exponential: its rounding to half can differ by an ulp here and there
     assert _rel(out.cpu().numpy(), _want(half, codes, cb16)) <= (1e-4 if silu else REL)
     assert float(zero.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("M", [4, 9, 16, 17, 33, 70, 200])
+@pytest.mark.parametrize("layout", ["tile", "fast"])
+@pytest.mark.parametrize("convention", ["slow", "fast"])
+def test_same_as_the_plane_kernels(M, layout, convention):
+    """The path that the library picks against the fp8-plane kernels, over layouts, sign conventions and results that
+    are written or added.  Each is within 1e-6 of the exact product (the planes 8e-7, the halves 6.2e-7)."""
+    N, K = 800, 672
+    x, codes, cb16 = _case(M, N, K, 9, "synthetic")
+    codes = _dev(codes)
+    packed = dmm.fast_pack(codes) if layout == "fast" else dmm.transpose_tile(codes)
+    kw = dict(layout=_lib.LAYOUT_FAST if layout == "fast" else _lib.LAYOUT_TILE,
+              sign_convention=_lib.SIGN_FAST if convention == "fast" else _lib.SIGN_SLOW)
+    base = torch.randn((M, N), device="cuda")
+    for accumulate, atomic in ((False, False), (True, False), (True, True)):
+        got = []
+        for path in (_lib.PATH_AUTO, _lib.PATH_TCGEN05_F8):
+            out = base.clone()
+            dmm.decode_matmul_fp16(_dev(x), packed, _dev(cb16), 0.5, out, path=path, accumulate=accumulate, atomic=atomic, **kw)
+            got.append(out.cpu().numpy())
+        assert _rel(got[0], got[1].astype(np.float64)) <= 2e-6
+
+
+def test_wide_rows_of_a_larger_buffer():
+    """Rows of x that lie further apart than K (fp16 and fp32), as a layer reads a part of the one before."""
+    M, N, K, ld = 40, 288, 544, 800
+    x, codes, cb16 = _case(M, N, ld, 10)
+    codes = np.ascontiguousarray(codes[:, : K // 8])
+    want = _want(np.ascontiguousarray(x[:, :K]), codes, cb16)
+    tiled, cb = _dev(o.tile_pack(codes)), _dev(cb16)
+    for t, kind in ((_dev(x), _lib.X_F16), (_dev(x.astype(np.float32)), _lib.X_F32)):
+        out = torch.empty((M, N), device="cuda")
+        dmm.decode_matmul_fused(t, tiled, cb, 1.0, out, x_kind=kind)
+        assert _rel(out.cpu().numpy(), want) <= REL
 
 
 def test_small_workspace_leaves_the_tiles_whole():
