@@ -2,8 +2,8 @@
 // one launch per product.  Same data path as the kernel of dmm_umma.cuh (read that header first) with a
 // different division of labour around it: one TMA producer per decoder group, activations staged in
 // fixed "rounds" so that an MMA issuer finds its operands by increments, leaner issuer loops.  The
-// library uses it for 17 to 32 batch rows, where the single in-order issuer pair of the first kernel
-// is the limit.
+// library uses it for 17 to 32 batch rows on planes (large fused steps, tensor-parallel forms), where the
+// single in-order issuer pair of the first kernel is the limit.
 //
 // Decoded weights are the A operand of tcgen05.mma and live only in tensor memory: a decoder
 // thread owns two output rows, decodes their codes in registers (two table look-ups and two XORs

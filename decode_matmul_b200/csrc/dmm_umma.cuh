@@ -6,7 +6,7 @@
 // the canonical no-swizzle K-major layout; accumulators live in TMEM.
 //
 // Operand policies that share the kernel:
-//   PolF8   fp16 family, what the library picks.  Weights as fp6 E2M3 bytes (sign << 5 | |q|,
+//   PolF8   fp16 family, small batches and large fused steps (dmm_wide.cuh has the rest).  Weights as fp6 E2M3 bytes (sign << 5 | |q|,
 //           value q/8: exact, and produced by the table XOR alone, 7 instructions per code),
 //           the fp16 activations split EXACTLY into four E5M2 planes (the top byte of the half,
 //           then of the remainder, ...), kind::f8f6f4, K = 32.  The planes are stacked along
@@ -20,11 +20,12 @@
 //   PolF16  fp16 family, fp16 operands (DMM_PATH_TCGEN05): weights as fp16 integers q (byte ->
 //           half by magic number), activations as fp16, kind::f16, K = 16.  A cross-check.
 //   PolF8Fast / PolI8Fast: the same over codes in the layout of fast_decode_matmul_cuda.
+//   PolF8Long: PolF8 with one hand-over per four k-tiles (16 and 64 columns).
 // Template flags: kChain (several dependent products in one cooperative launch, the CTAs stay
 // resident), kTp (tensor-parallel forms: epilogue that adds into every rank's buffer, producer
 // and consumer of the slots form) and kSplit (four TMA producer warps, batch 1 and 2).
 // Companions in this file: planes_kernel, xrank_barrier_kernel, xrank_allreduce_kernel,
-// tp_finalize_kernel.  Batch 17..32 of the fp16 family runs on dmm_kernel (dmm_tc.cuh).
+// tp_finalize_kernel.  Batch 17..32 on planes runs on dmm_kernel (dmm_tc.cuh).
 //
 // Work decomposition.  A super-tile is 16 strips = 256 output rows = two M=128 MMA tiles:
 // tile 0 holds strip rows 0..7 (h = 0) and tile 1 strip rows 8..15 (h = 1) of the 16 strips,
@@ -204,6 +205,15 @@ struct PolF8 {
     static constexpr int kACols = 8;   // TMEM columns of one k-tile of one MMA tile (32 k x 1 byte)
     static constexpr uint32_t x_tile_bytes(int) { return 1024; }  // 2 k-halves x (4 planes x 8 rows) x 16 B
     static constexpr int out_cols(int nmma) { return nmma / 4; }    // batch columns per launch: 8 or 16
+};
+// The same with one hand-over per four k-tiles instead of two, in one group buffer of twice the size: half the waits,
+// fences, arrivals and commits per tile, and the decoders, which are short of issue slots, gain it.  A block of the
+// 70B stack at batch 1 70.5 us (72.5 with PolF8), at 2 77.9 (79.8), at 16 105.5 (112.5).  Not for the
+// 32-column build, whose single accumulator set has nothing to hide the longer hand-over at the end of a segment
+// behind (batch 4: 90.7 against 85.3), nor for int8 (4096 x 4096: 8.0 against 7.6).
+struct PolF8Long : PolF8 {
+    static constexpr int kG = 4;
+    static constexpr int kNA = 1;
 };
 // Integer family (the reference's own operator: int8 activations, int32 result, exact): the
 // structure of the fp8 policy -- epoch-resident activations, four accumulator sets -- with the
@@ -837,35 +847,45 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
                 for (int g0 = 0; g0 < n; g0 += G) {
                     const int buf = static_cast<int>(sA % NA);
                     const int sl = q * NA + buf;
-                    if (sA >= NA) mbar_wait(bar(Plan::kBarFree + sl), ((sA / NA) - 1) & 1, flags);
-                    tc_fence_after();
                     const uint32_t acol = tlane + Plan::kDCols + static_cast<uint32_t>(sl) * Plan::kBufCols;
+                    auto wait_free = [&] {
+                        if (sA >= NA) mbar_wait(bar(Plan::kBarFree + sl), ((sA / NA) - 1) & 1, flags);
+                        tc_fence_after();
+                    };
                     if constexpr (Pol::kIsF8) {
-                        // group buffer columns: [tile][k-tile][8]; two k-tiles -> one x16 store per tile
-                        uint32_t r0[8 * G], r1[8 * G];
+                        // group buffer columns: [tile][k-tile][8]; two k-tiles at a time -> one x16 store per tile
 #pragma unroll
-                        for (int i = 0; i < G; ++i) {
-                            uint4 cw = make_uint4(0, 0, 0, 0);
-                            if (g0 + i < n) cw = fast ? fetch_fast_ktile(fsrc, C, wq, lane, g0 + i) : lds128(src + (g0 + i) * 128);
-                            const uint32_t w[4] = {cw.x, cw.y, cw.z, cw.w};
+                        for (int h0 = 0; h0 < G; h0 += 2) {
+                            if (h0 > 0 && g0 + h0 >= n) break;
+                            if (NA > 1 && h0 == 0) wait_free();
+                            uint32_t r0[16], r1[16];
 #pragma unroll
-                            for (int t = 0; t < 4; ++t) {
-                                uint2 d0, d1;
-                                if constexpr (Pol::kIsInt) {
-                                    d0 = decode8<0>(w[t], ll);
-                                    d1 = decode8<1>(w[t], ll);
-                                } else {
-                                    d0 = decode8_fp6<0>(w[t], ll);
-                                    d1 = decode8_fp6<1>(w[t], ll);
+                            for (int i = 0; i < 2; ++i) {
+                                const int kt = g0 + h0 + i;
+                                uint4 cw = make_uint4(0, 0, 0, 0);
+                                if (kt < n) cw = fast ? fetch_fast_ktile(fsrc, C, wq, lane, kt) : lds128(src + kt * 128);
+                                const uint32_t w[4] = {cw.x, cw.y, cw.z, cw.w};
+#pragma unroll
+                                for (int t = 0; t < 4; ++t) {
+                                    uint2 d0, d1;
+                                    if constexpr (Pol::kIsInt) {
+                                        d0 = decode8<0>(w[t], ll);
+                                        d1 = decode8<1>(w[t], ll);
+                                    } else {
+                                        d0 = decode8_fp6<0>(w[t], ll);
+                                        d1 = decode8_fp6<1>(w[t], ll);
+                                    }
+                                    r0[8 * i + 2 * t] = d0.x; r0[8 * i + 2 * t + 1] = d0.y;
+                                    r1[8 * i + 2 * t] = d1.x; r1[8 * i + 2 * t + 1] = d1.y;
                                 }
-                                r0[8 * i + 2 * t] = d0.x; r0[8 * i + 2 * t + 1] = d0.y;
-                                r1[8 * i + 2 * t] = d1.x; r1[8 * i + 2 * t + 1] = d1.y;
                             }
+                            // (one buffer per group: the first two k-tiles are decoded before it is waited for)
+                            if (NA == 1 && h0 == 0) wait_free();
+                            tmem_st16(acol + h0 * Pol::kACols, r0);
+                            tmem_st16(acol + (G + h0) * Pol::kACols, r1);
                         }
-                        static_assert(G == 2 || !Pol::kIsF8, "fp8 policy stores two k-tiles at once");
-                        tmem_st16(acol, reinterpret_cast<const uint32_t(&)[16]>(r0));
-                        tmem_st16(acol + G * Pol::kACols, reinterpret_cast<const uint32_t(&)[16]>(r1));
                     } else {
+                        wait_free();
                         const uint4 cw = lds128(src + g0 * 128);
                         const uint32_t w[4] = {cw.x, cw.y, cw.z, cw.w};
                         uint32_t r0[16], r1[16];
@@ -1798,9 +1818,9 @@ inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cuda
         // up to two batch rows all four planes fit one 8-row core matrix: 16 MMA columns instead of 32 halve
         // what the tensor core reads from shared memory per MMA (the build with four TMA producers).  For 3
         // and 4 rows (two core matrices of the dense planes) it measured 1-2 % faster but cost batch 2 3 %.
-        if (p.M <= 2) return launch_umma_one<PolF8, 16>(p, num_sms, pdl, stream);
+        if (p.M <= 2) return launch_umma_one<PolF8Long, 16>(p, num_sms, pdl, stream);
         if (p.M <= 8) return launch_umma_one<PolF8, 32>(p, num_sms, pdl, stream);
-        if (p.M <= 16) return launch_umma_one<PolF8, 64>(p, num_sms, pdl, stream);
+        if (p.M <= 16) return launch_umma_one<PolF8Long, 64>(p, num_sms, pdl, stream);
         return launch_umma_one<PolF8, 128>(p, num_sms, pdl, stream);
     }
     if (p.M <= 16) return launch_umma_one<PolF16, 16>(p, num_sms, pdl, stream);
