@@ -343,7 +343,8 @@ size_t dmm_workspace_bytes(int64_t M, int64_t N, int64_t K);
  */
 int dmm_status(unsigned *status_out);
 
-/* Which path DMM_PATH_AUTO resolves to for this shape (one of the DMM_PATH_* values above). */
+/* Which path DMM_PATH_AUTO resolves to for this shape (one of the DMM_PATH_* values above; larger batches run on the
+   fp16-operand kernel that only DMM_PATH_AUTO takes, see DMM_PATH_TCGEN05_F8). */
 int dmm_select_path(int64_t M, int64_t N, int64_t K);
 
 /* Number of kernels the library has launched in this process (all devices, all entry points). */
