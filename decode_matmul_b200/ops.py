@@ -149,40 +149,70 @@ def decode_matmul_fused(x, weights_compressed, codebook_fp16, scale, output, *, 
     return output
 
 
+def _check_on(t: torch.Tensor, name: str, dtype: torch.dtype, index: int) -> None:
+    """``_check_input``, and that the tensor is on CUDA device ``index``."""
+    if isinstance(t, torch.Tensor) and t.get_device() == index and t.dtype is dtype and t.is_contiguous():
+        return
+    _check_input(t, name, dtype)
+    _req(False, f"{name} is on device {t.get_device()}, not on {index}")
+
+
 def fused_op(x, lin, output, *, x_kind=_lib.X_F32, x_gap=0, zero=None) -> tuple:
     """One product of :func:`decode_matmul_sequence`: the arguments of :func:`decode_matmul_fused` with ``lin`` a
-    layer (codes, codebook, scale)."""
+    layer (codes, codebook, scale).  What comes back is (the fields of ``dmm_fused_op``, rows, device index, the
+    tensors): addresses of what the checks have seen, and the tensors themselves so that the memory stays theirs until
+    the product has been launched."""
     codes, cb = lin.codes, lin.codebook
     _check_input(x, "x", torch.float16 if x_kind == _lib.X_F16 else torch.float32)
-    _check_input(codes, "weights_compressed", torch.int16)
-    _check_input(cb, "codebook_fp16", torch.float16)
-    _check_input(output, "output", torch.float32)
-    _req(x.dim() == 2 and codes.dim() == 2, "x and weights_compressed must be 2-D")
+    index = x.get_device()
+    _check_on(codes, "weights_compressed", torch.int16, index)
+    _check_on(cb, "codebook_fp16", torch.float16, index)
+    _check_on(output, "output", torch.float32, index)
+    if x.dim() != 2 or codes.dim() != 2:
+        raise RuntimeError("x and weights_compressed must be 2-D")
+    if cb.numel() != 2048:
+        raise RuntimeError("codebook_fp16 must have shape [256, 8]")
     M, ld = x.shape
     N, k8 = codes.shape
-    _req(ld >= 8 * k8, "x rows are shorter than the reduction length")
-    _req(output.shape == (M, N), "output must have shape [M, N]")
+    if ld < 8 * k8:
+        raise RuntimeError("x rows are shorter than the reduction length")
+    if output.shape != (M, N):
+        raise RuntimeError("output must have shape [M, N]")
     if zero is not None:
-        _check_input(zero, "zero", torch.float32)
-    return (x.data_ptr(), x_kind, ld, x_gap, codes.data_ptr(), cb.data_ptr(), lin.scale, output.data_ptr(), N, 8 * k8,
-            None if zero is None else zero.data_ptr(), 0 if zero is None else zero.numel())
+        _check_on(zero, "zero", torch.float32, index)
+    fields = (x.data_ptr(), x_kind, ld, x_gap, codes.data_ptr(), cb.data_ptr(), lin.scale, output.data_ptr(), N, 8 * k8,
+              None if zero is None else zero.data_ptr(), 0 if zero is None else zero.numel())
+    return fields, M, index, (x, codes, cb, output, zero)
 
 
 def decode_matmul_sequence(ops, M, device, *, next_weights=None, sign_convention=_lib.SIGN_SLOW, pdl=True, workspace=None):
     """Dependent products one after the other (``dmm_f16_sequence``): every op, a :func:`fused_op` over M rows, ADDS
     its product to its output with atomic adds, and each launch is told which weights the next one streams
     (``next_weights``: a layer that follows the last op).  One call into the library for all of them."""
-    arr = (_lib.FusedOp * len(ops))(*ops)
+    current = torch.cuda.current_device()
+    index = (device if isinstance(device, torch.device) else torch.device(device)).index
+    if index is None:
+        index = current
+    fields = []
+    for args, rows, at, _ in ops:
+        if rows != M or at != index:
+            raise RuntimeError(f"an op has {rows} rows on device {at}, not {M} on device {index}")
+        fields.append(args)
+    arr = (_lib.FusedOp * len(fields))(*fields)
     nxt = (None, 0, 0)
     if next_weights is not None:
-        n, k8 = next_weights.codes.shape
-        nxt = (next_weights.codes.data_ptr(), n, 8 * k8)
+        codes = next_weights.codes
+        _check_on(codes, "next_weights", torch.int16, index)
+        n, k8 = codes.shape
+        nxt = (codes.data_ptr(), n, 8 * k8)
+    if workspace is not None and not (workspace.get_device() == index and workspace.is_contiguous()):
+        raise RuntimeError(f"workspace must be contiguous, on device {index}")
     flags = _lib.FLAG_ACCUMULATE | _lib.FLAG_ATOMIC | (_lib.FLAG_PDL if pdl else 0)
-    with torch.cuda.device(device):
-        rc = _lib.lib().dmm_f16_sequence(arr, len(ops), M, sign_convention, flags, *nxt,
+    with _SAME_DEVICE if index == current else torch.cuda.device(index):
+        rc = _lib.lib().dmm_f16_sequence(arr, len(fields), M, sign_convention, flags, *nxt,
                                          None if workspace is None else workspace.data_ptr(),
                                          0 if workspace is None else workspace.numel() * workspace.element_size(),
-                                         _stream_ptr(device))
+                                         torch._C._cuda_getCurrentRawStream(index))
     _lib.check(rc, "decode_matmul_sequence")
 
 

@@ -1,0 +1,33 @@
+"""decode_matmul_sequence on the GPU: the same as its products one by one."""
+import pytest
+import torch
+
+import decode_matmul_b200 as dmm
+from decode_matmul_b200 import _lib, ops
+from decode_matmul_b200.linear import DecodeLinear
+from oracle import dmm_oracle as o
+
+pytestmark = pytest.mark.gpu
+
+
+def _layers(shapes):
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    cb = torch.from_numpy(o.synthetic_codebook(42)).cuda()
+    return [DecodeLinear(torch.randint(-32768, 32768, (n, k // 8), dtype=torch.int16, device="cuda", generator=gen), cb, 2.0 ** -7)
+            for n, k in shapes]
+
+
+@pytest.mark.parametrize("M", [1, 5, 16, 24])
+def test_same_as_the_products_one_by_one(M):
+    first, second = _layers([(544, 1056), (1056, 544)])
+    x = torch.randn((M, 1056), device="cuda")
+    a, y = torch.zeros((M, 544), device="cuda"), torch.zeros((M, 1056), device="cuda")
+    ops.decode_matmul_sequence([ops.fused_op(x, first, a), ops.fused_op(a, second, y)], M, x.device)
+    a1 = torch.zeros_like(a)
+    dmm.decode_matmul_fused(x, first.codes, first.codebook, first.scale, a1, accumulate=True, atomic=True)
+    y1 = torch.zeros_like(y)
+    dmm.decode_matmul_fused(a, second.codes, second.codebook, second.scale, y1, accumulate=True, atomic=True)
+    # the same kernels over the same inputs: only the order of the atomic adds differs, a few roundings of 2^-24
+    for got, want in ((a, a1), (y, y1)):
+        assert float((got - want).norm() / want.norm()) <= 4 * 2.0 ** -24
+    assert dmm.status() == 0
