@@ -861,9 +861,12 @@ int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_con
     if (n_ops < 1) return DMM_ERR_ARG;
     for (int i = 0; i < n_ops; ++i) {
         const dmm_fused_op &op = ops[i];
-        const bool last = i + 1 == n_ops;
-        int rc = last ? dmm_hint_next_weights(next_codes, next_N, next_K)
-                      : dmm_hint_next_weights(ops[i + 1].codes, ops[i + 1].N, ops[i + 1].K);
+        int rc = 0;
+        if (i + 1 == n_ops) {
+            rc = dmm_hint_next_weights(next_codes, next_N, next_K);
+        } else if (dmm_hint_next_weights(ops[i + 1].codes, ops[i + 1].N, ops[i + 1].K) != 0) {
+            t_next_hint = NextHint();  // that op's own call will refuse it; this one is launched all the same
+        }
         if (rc == 0)
             rc = dmm_f16_fused(op.x, op.x_kind, op.x_ld, op.x_gap, op.codes, op.cb16, op.scale, op.out, M, op.N, op.K,
                                sign_convention, DMM_LAYOUT_TILE, DMM_PATH_AUTO, flags, op.zero_ptr, op.zero_count, workspace,

@@ -257,7 +257,8 @@ int dmm_f16_chain(const dmm_chain_op *ops, int n_ops, const void *cb16, int64_t 
  * follows, and next_codes / next_N / next_K (may be null / 0) for what follows the last one.  The
  * same launches as n_ops calls would make, for programs whose small products take less time on the GPU than
  * a call from their language does.  flags, workspace and stream as in dmm_f16_fused.  On an error the call
- * returns at once: the ops before the one that failed have been launched.
+ * returns at once: the ops before the one that was refused have been launched, no later one has.  A next_codes that
+ * dmm_hint_next_weights refuses is an error of the last op.
  */
 typedef struct dmm_fused_op {
     const void *x;        /* activations of this op, see x_kind */

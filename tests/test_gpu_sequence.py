@@ -1,4 +1,4 @@
-"""decode_matmul_sequence on the GPU: the same as its products one by one."""
+"""decode_matmul_sequence on the GPU: the same as its products one by one, and what an error leaves behind."""
 import pytest
 import torch
 
@@ -30,4 +30,31 @@ def test_same_as_the_products_one_by_one(M):
     # the same kernels over the same inputs: only the order of the atomic adds differs, a few roundings of 2^-24
     for got, want in ((a, a1), (y, y1)):
         assert float((got - want).norm() / want.norm()) <= 4 * 2.0 ** -24
+    assert dmm.status() == 0
+
+
+def test_an_error_in_the_middle():
+    """The ops before the refused one have been launched, the ones behind it have not, and no hint is left for the next
+    call."""
+    good, last = _layers([(544, 1056), (1056, 544)])
+    M = 2
+    x = torch.randn((M, 1056), device="cuda")
+    a, y = torch.zeros((M, 544), device="cuda"), torch.full((M, 1056), 3.0, device="cuda")
+    bad = _layers([(48, 544)])[0]
+    bad.codes = bad.codes[:24].contiguous()  # 24 rows: not a multiple of 16
+    block = [ops.fused_op(x, good, a), ops.fused_op(a, bad, torch.zeros((M, 24), device="cuda")), ops.fused_op(a, last, y)]
+    with pytest.raises(RuntimeError, match="decode_matmul_sequence"):
+        ops.decode_matmul_sequence(block, M, x.device)
+    want = torch.zeros_like(a)
+    dmm.decode_matmul_fused(x, good.codes, good.codebook, good.scale, want, accumulate=True, atomic=True)
+    assert float((a - want).norm() / want.norm()) <= 4 * 2.0 ** -24
+    assert bool((y == 3.0).all())
+    # an op in the middle whose codes are missing altogether, through the C entry
+    arr = (_lib.FusedOp * 2)(block[0][0], block[2][0])
+    arr[1].codes = None
+    a.zero_()
+    rc = _lib.lib().dmm_f16_sequence(arr, 2, M, _lib.SIGN_SLOW, _lib.FLAG_ACCUMULATE | _lib.FLAG_ATOMIC, None, 0, 0, None, 0,
+                                     torch.cuda.current_stream().cuda_stream)
+    assert rc == -1
+    assert float((a - want).norm() / want.norm()) <= 4 * 2.0 ** -24
     assert dmm.status() == 0
