@@ -53,14 +53,17 @@ static int current_device_state(DeviceState **out) {
     return 0;
 }
 
-// Size of the library's own workspace on first use: tickets for N up to 2^24 (4 MiB) and behind them either the
+// Size of the library's own workspace on first use: the tickets and behind them either the
 // partial tiles of the wide kernel (148 CTAs, 128 columns: 37 MiB) or stream-K partials at batch 64 (up to
 // 256 CTAs: 16 MiB) and the activation planes for K up to 2^17 (16 MiB).
 constexpr size_t kDefaultWorkspace = size_t(42) << 20;
 
-static size_t ticket_bytes(long long N) {
-    const size_t b = static_cast<size_t>(N / 16) * sizeof(unsigned);
-    return (b + 255) & ~static_cast<size_t>(255);
+// Counters of the split tiles, at the start of every workspace: one per CTA.  A split tile counts at the index of the
+// first CTA that has a part of it, whose own range ends inside the tile, so no two tiles share a counter.  The block has
+// the same size for every shape: calls of different shapes share a workspace, and the partial sums that one leaves
+// must not lie where another expects its counters to be zero.
+static size_t ticket_bytes(int num_sms) {
+    return (static_cast<size_t>(num_sms) * sizeof(unsigned) + 255) & ~static_cast<size_t>(255);
 }
 
 // Every path shares the ticket block; the partial block is sized for the widest path
@@ -72,8 +75,8 @@ static size_t partial_bytes(long long M, int num_sms) {
     if (umma > per_slot) per_slot = umma;
     return static_cast<size_t>(num_sms) * 2 * per_slot * 4;
 }
-static size_t planes_offset(long long M, long long N, int num_sms) {
-    return (ticket_bytes(N) + partial_bytes(M, num_sms) + 255) & ~static_cast<size_t>(255);
+static size_t planes_offset(long long M, int num_sms) {
+    return (ticket_bytes(num_sms) + partial_bytes(M, num_sms) + 255) & ~static_cast<size_t>(255);
 }
 // Which kernel a product of the fp16 family runs on: the wide one (dmm_wide.cuh) or the fp8-plane kernels.  Per
 // tile of codes (256 rows x 32 k) and SM the wide kernel costs more up to some 32 rows, per call it costs less (no
@@ -89,16 +92,16 @@ static bool wide_is_faster(long long M, long long N, long long K, bool fused, in
     return M > 16 || (M >= 4 && per_sm <= 15 * M - 28);
 }
 
-static size_t workspace_need(long long M, long long N, long long K, int num_sms) {
-    return planes_offset(M, N, num_sms) + static_cast<size_t>(K) * 128;
+static size_t workspace_need(long long M, long long K, int num_sms) {
+    return planes_offset(M, num_sms) + static_cast<size_t>(K) * 128;
 }
 
 // Returns the workspace to use: the caller's (checked for size) or the library's own,
 // grown on demand.  The ticket counters must be zero before the first launch; the
 // library's buffer is cleared when it is (re)allocated, a caller's buffer by the caller.
-static int resolve_workspace(DeviceState *d, long long M, long long N, long long K, void *user, size_t user_bytes,
+static int resolve_workspace(DeviceState *d, long long M, long long K, void *user, size_t user_bytes,
                              cudaStream_t stream, void **ws, size_t *ws_bytes = nullptr) {
-    const size_t need = workspace_need(M, N, K, d->num_sms);
+    const size_t need = workspace_need(M, K, d->num_sms);
     if (user != nullptr) {
         if (user_bytes < need) return DMM_ERR_WORKSPACE;
         if (reinterpret_cast<uintptr_t>(user) % 256 != 0) return DMM_ERR_ALIGN;
@@ -182,7 +185,7 @@ static int run_stream(int family, const void *x, const void *codes, const void *
     int rc = current_device_state(&d);
     if (rc) return rc;
     void *ws = nullptr;
-    rc = resolve_workspace(d, M, N, K, workspace, workspace_bytes, stream, &ws);
+    rc = resolve_workspace(d, M, K, workspace, workspace_bytes, stream, &ws);
     if (rc) return rc;
     const size_t x_elem = family == 0 ? 1 : 2;
     for (long long m0 = 0; m0 < M; m0 += 16) {
@@ -192,7 +195,7 @@ static int run_stream(int family, const void *x, const void *codes, const void *
         p.cb = cb;
         p.out = reinterpret_cast<uint8_t *>(out) + static_cast<size_t>(m0) * N * 4;
         p.tickets = reinterpret_cast<unsigned *>(ws);
-        p.partials = reinterpret_cast<uint8_t *>(ws) + ticket_bytes(N);
+        p.partials = reinterpret_cast<uint8_t *>(ws) + ticket_bytes(d->num_sms);
         p.M = M - m0 < 16 ? M - m0 : 16;
         p.N = N;
         p.K = K;
@@ -219,7 +222,7 @@ static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, 
     if (rc) return rc;
     void *ws = nullptr;
     size_t ws_bytes = 0;
-    rc = resolve_workspace(d, M, N, K, workspace, workspace_bytes, stream, &ws, &ws_bytes);
+    rc = resolve_workspace(d, M, K, workspace, workspace_bytes, stream, &ws, &ws_bytes);
     if (rc) return rc;
     const bool pdl = (flags & DMM_FLAG_PDL) != 0;
     const long long step = x_kind == DMM_X_F16 ? M : 64;
@@ -227,12 +230,12 @@ static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, 
     for (long long m0 = 0; m0 < M; m0 += step) {
         const long long rows = M - m0 < step ? M - m0 : step;
         const uint8_t *xm = reinterpret_cast<const uint8_t *>(x) + static_cast<size_t>(m0) * x_ld * (x_kind == DMM_X_F16 ? 2 : 4);
-        size_t capacity = ws_bytes - ticket_bytes(N);
+        size_t capacity = ws_bytes - ticket_bytes(d->num_sms);
         long long ld = x_ld;
         int mode = x_kind;
         if (x_kind != DMM_X_F16 && rows > kWConvRows) {
-            uint8_t *half = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, N, d->num_sms);
-            capacity = planes_offset(M, N, d->num_sms) - ticket_bytes(N);
+            uint8_t *half = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, d->num_sms);
+            capacity = planes_offset(M, d->num_sms) - ticket_bytes(d->num_sms);
             rc = launch_half(xm, x_kind, x_ld, x_gap, static_cast<int>(rows), K, half, pdl, stream);
             g_launches.fetch_add(1, std::memory_order_relaxed);
             if (rc) return rc;
@@ -244,7 +247,7 @@ static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, 
         p.cb = cb16;
         p.out = out + static_cast<size_t>(m0) * N;
         p.tickets = reinterpret_cast<unsigned *>(ws);
-        p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ws) + ticket_bytes(N));
+        p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ws) + ticket_bytes(d->num_sms));
         p.M = rows;
         p.N = N;
         p.scale = scale;
@@ -255,8 +258,7 @@ static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, 
             p.zero_ptr = zero_ptr;
             p.zero_count = zero_count;
         }
-        rc = launch_wide(p, xm, mode, ld, x_gap, codes, K, fast_layout, capacity, static_cast<long long>(ticket_bytes(N) / sizeof(unsigned)), d->num_sms,
-                         pdl, stream);
+        rc = launch_wide(p, xm, mode, ld, x_gap, codes, K, fast_layout, capacity, d->num_sms, pdl, stream);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (rc) return rc;
     }
@@ -287,7 +289,7 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
     int rc = current_device_state(&d);
     if (rc) return rc;
     void *ws = nullptr;
-    rc = resolve_workspace(d, M, N, K, workspace, workspace_bytes, stream, &ws);
+    rc = resolve_workspace(d, M, K, workspace, workspace_bytes, stream, &ws);
     if (rc) return rc;
     if (may_go_wide && wide_is_faster(M, N, K, x_kind != DMM_X_F16 || (flags & DMM_FLAG_ATOMIC) != 0, d->num_sms))
         return run_wide(x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K, sign_convention, flags, workspace,
@@ -300,7 +302,7 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
         p.M = M - m0 < step ? M - m0 : step;
         if (f8 && p.M >= kPlanesMinBatch && !(tp != nullptr && tp->mode == 3)) {
             // split the activations into E5M2 planes once, instead of once per CTA inside the kernel
-            uint8_t *planes = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, N, d->num_sms);
+            uint8_t *planes = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, d->num_sms);
             rc = launch_planes(p.x, x_kind, x_ld, x_gap, static_cast<int>(p.M), K, planes, pdl, stream);
             g_launches.fetch_add(1, std::memory_order_relaxed);
             if (rc) return rc;
@@ -313,7 +315,7 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
         p.cb = cb16;
         p.out = out + static_cast<size_t>(m0) * N;
         p.tickets = reinterpret_cast<unsigned *>(ws);
-        p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ws) + ticket_bytes(N));
+        p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ws) + ticket_bytes(d->num_sms));
         p.N = N;
         p.K = K;
         // accumulators hold sum(x * q / 8) (fp6 weights) or sum(x * q) (fp16 weights); weight = q / 4
@@ -370,7 +372,7 @@ static int run_umma_i8(const void *x, const void *codes, const void *cb64, int32
     int rc = current_device_state(&d);
     if (rc) return rc;
     void *ws = nullptr;
-    rc = resolve_workspace(d, M, N, K, workspace, workspace_bytes, stream, &ws);
+    rc = resolve_workspace(d, M, K, workspace, workspace_bytes, stream, &ws);
     if (rc) return rc;
     // Integer sums do not depend on their order, so partial super-tiles are always added with
     // atomics (no workspace round trip, no ticket); a plain product clears the output first.
@@ -386,7 +388,7 @@ static int run_umma_i8(const void *x, const void *codes, const void *cb64, int32
         p.cb = cb64;
         p.out = reinterpret_cast<float *>(out + static_cast<size_t>(m0) * N);  // int32 behind the kernel's generic pointer
         p.tickets = reinterpret_cast<unsigned *>(ws);
-        p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ws) + ticket_bytes(N));
+        p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ws) + ticket_bytes(d->num_sms));
         p.M = M - m0 < 32 ? M - m0 : 32;
         p.N = N;
         p.K = K;
@@ -409,7 +411,7 @@ static int run_umma_i8(const void *x, const void *codes, const void *cb64, int32
 // ---------------------------------------------------------------------------------------
 constexpr int kNoAllocMaxCtas = 160;
 constexpr long long kNoAllocMaxM = 8;
-constexpr long long kNoAllocMaxN = 262144;  // 1024 super-tiles -> 4 KiB of tickets
+constexpr long long kNoAllocMaxN = 262144;
 constexpr size_t kNoAllocTicketBytes = 4096;
 constexpr size_t kNoAllocBytes = kNoAllocTicketBytes + static_cast<size_t>(kNoAllocMaxCtas) * 2 * 2048 * sizeof(float);
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -824,9 +826,9 @@ size_t dmm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
     DeviceState *d = nullptr;
     int sms = 256;
     if (current_device_state(&d) == 0 && d->num_sms > 0) sms = d->num_sms;
-    size_t need = workspace_need(M, N, K, sms);
+    size_t need = workspace_need(M, K, sms);
     if (M > 64) {  // (with less the wide kernel leaves the last tiles whole)
-        const size_t wide = ticket_bytes(N) + wide_partial_bytes(M, sms);
+        const size_t wide = ticket_bytes(sms) + wide_partial_bytes(M, sms);
         if (wide > need) need = wide;
     }
     return need;

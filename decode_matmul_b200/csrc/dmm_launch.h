@@ -12,7 +12,7 @@ struct StreamParams {
     const void *cb;         // cb64 or cb16
     void *out;              // [M, N] int32 or fp32
     void *partials;         // workspace: [grid][2][S*MB*128] accumulator values
-    unsigned *tickets;      // workspace: one counter per super-strip, zero between launches
+    unsigned *tickets;      // workspace, see ticket_bytes in dmm_api.cu, zero between launches
     long long M, N, K;
     float scale;            // fp16 family only (already includes the 1/4 of quarter units)
     int accumulate;

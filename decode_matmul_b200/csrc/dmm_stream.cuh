@@ -298,9 +298,9 @@ __global__ void __launch_bounds__(kStreamWarps * 32, 1) stream_kernel(const Stre
             const long long c_lo = part_owner(T, G, ss_a), c_hi = part_owner(T, G, ss_b - 1);
             if (tid == 0) {
                 const unsigned expected = static_cast<unsigned>(c_hi - c_lo + 1);
-                const unsigned old = atomicAdd(p.tickets + ss, 1u);
+                const unsigned old = atomicAdd(p.tickets + c_lo, 1u);
                 const int last = old == expected - 1;
-                if (last) p.tickets[ss] = 0;  // ready for the next launch
+                if (last) p.tickets[c_lo] = 0;  // ready for the next launch
                 flags[1] = last;
             }
             __syncthreads();

@@ -357,9 +357,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) dmm_kernel(const __grid_constan
                     const int c_lo = part32_owner(p.part, ss_a), c_hi = part32_owner(p.part, ss_a + KT - 1);
                     if (ptid == 0) {
                         const unsigned expected = static_cast<unsigned>(c_hi - c_lo + 1);
-                        const unsigned old = atomicAdd(p.tickets + ss, 1u);
+                        const unsigned old = atomicAdd(p.tickets + c_lo, 1u);
                         const int last = old == expected - 1;
-                        if (last) p.tickets[ss] = 0;
+                        if (last) p.tickets[c_lo] = 0;
                         flags[1] = last;
                     }
                     named_barrier(2, 256);

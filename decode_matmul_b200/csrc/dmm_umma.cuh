@@ -344,7 +344,7 @@ struct UmmaParams {
     const void *cb;      // fp16 [256, 8]
     float *out;          // [M, N]
     float *partials;     // workspace [grid][2][kPartial]
-    unsigned *tickets;   // workspace, one per super-tile, zero between launches
+    unsigned *tickets;   // workspace, see ticket_bytes in dmm_api.cu, zero between launches
     long long M, N, K;
     int x_mode;
     long long x_ld, x_gap;  // row stride of x in elements; offset of the second operand (mode 2)
@@ -1028,9 +1028,9 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
                     const int c_lo = part32_owner(p.part, ss_a), c_hi = part32_owner(p.part, ss_a + KT - 1);
                     if (ptid == 0) {
                         const unsigned expected = static_cast<unsigned>(c_hi - c_lo + 1);
-                        const unsigned old = atomicAdd(p.tickets + ss, 1u);
+                        const unsigned old = atomicAdd(p.tickets + c_lo, 1u);
                         const int last = old == expected - 1;
-                        if (last) p.tickets[ss] = 0;
+                        if (last) p.tickets[c_lo] = 0;
                         flags[1] = last;
                     }
                     named_barrier(2, 256);

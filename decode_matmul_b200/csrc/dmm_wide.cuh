@@ -74,7 +74,7 @@ struct WideParams {
     const void *cb;     // fp16 [256, 8]
     float *out;         // [M, N]
     float *partials;    // workspace [grid][2][NB * 256]
-    unsigned *tickets;  // workspace, one per split tile, zero between launches
+    unsigned *tickets;  // workspace, see ticket_bytes in dmm_api.cu, zero between launches
     long long M, N;
     float scale;
     int accumulate, atomic_reduce, sign_convention;
@@ -431,9 +431,9 @@ __global__ void __launch_bounds__(kConv ? kWConvThreads : kWThreads, 1) wide_ker
                             const int a = prev.split * p.units;
                             const int c_lo = part32_owner(p.part, a), c_hi = part32_owner(p.part, a + p.units - 1);
                             if (tid == 0) {
-                                const unsigned old = atomicAdd(p.tickets + prev.split, 1u);
+                                const unsigned old = atomicAdd(p.tickets + c_lo, 1u);
                                 const int last = old == static_cast<unsigned>(c_hi - c_lo);
-                                if (last) p.tickets[prev.split] = 0;
+                                if (last) p.tickets[c_lo] = 0;
                                 flags[1] = last;
                             }
                             named_barrier(1, kWDecWarps * 32);
@@ -745,9 +745,9 @@ inline int launch_wide_as(WideArgs &args, unsigned grid, bool pdl, cudaStream_t 
 }
 
 // p carries cb, out, partials, tickets, M, N, scale, flags, sign convention and the buffer to clear; x is fp16
-// [M, K] with rows x_ld elements apart, or fp32 as x_mode says (at most kWConvRows rows).  partial_capacity: bytes of workspace behind p.partials; n_tickets: counters at p.tickets.
+// [M, K] with rows x_ld elements apart, or fp32 as x_mode says (at most kWConvRows rows).  partial_capacity: bytes of workspace behind p.partials.
 inline int launch_wide(WideParams p, const void *x, int x_mode, long long x_ld, long long x_gap, const void *codes, long long K, bool fast_layout,
-                       size_t partial_capacity, long long n_tickets, int num_sms, bool pdl, cudaStream_t stream) {
+                       size_t partial_capacity, int num_sms, bool pdl, cudaStream_t stream) {
     WideArgs args = {};
     p.nb = wide_cols(p.M);
     p.units = static_cast<int>((K + 127) / 128);
@@ -756,7 +756,7 @@ inline int launch_wide(WideParams p, const void *x, int x_mode, long long x_ld, 
     if (tiles * p.units >= (1ll << 31)) return DMM_ERR_SHAPE;
     long long whole = tiles / num_sms, rest = tiles - whole * num_sms;
     long long grid = whole > 0 ? num_sms : 0;
-    const bool can_split = p.atomic_reduce || (partial_capacity >= wide_partial_bytes(p.M, num_sms) && rest <= n_tickets);
+    const bool can_split = p.atomic_reduce || partial_capacity >= wide_partial_bytes(p.M, num_sms);
     if (rest > 0) {
         // How many CTAs share the remaining tiles: estimated cycles of the longest CTA.  A unit costs about
         // 640 + 10 nb, and a split tile a fix-up: its last CTA reads nb KiB per contributor at 64 bytes a cycle.
