@@ -80,16 +80,29 @@ static size_t planes_offset(long long M, int num_sms) {
 }
 // Which kernel a product of the fp16 family runs on: the wide one (dmm_wide.cuh) or the fp8-plane kernels.  Per
 // tile of codes (256 rows x 32 k) and SM the wide kernel costs more up to some 32 rows, per call it costs less (no
-// planes kernel, a cheaper fix-up), so the line is a number of tiles per SM.  Microseconds, planes / wide:
-//   fp16 in, own result   4 x 4096 x 4096 13.5 / 8.8, 4 x 28672 x 8192 26.6 / 34.6; 8 x 8192 x 8192 17.6 / 17.3, 8 x
-//                         57344 x 8192 45 / 62; 16 x 28672 x 8192 35.7 / 35.4, 16 x 57344 x 8192 55 / 62; from 17
-//                         rows on always (32 x 28672 x 8192 48 / 36)
-//   added into a stack    a block of the 7B model at 16 rows 57.8 / 51.7, at 24 69.9 / 60.7; of the 70B model at 16
-//                         112 / 148, at 24 137 / 147; from 33 rows on the planes take two passes
-static bool wide_is_faster(long long M, long long N, long long K, bool fused, int num_sms) {
+// planes kernel, a cheaper fix-up), so the line is a number of tiles per SM, t.  Microseconds on the GPU (CUDA graph over
+// several matrices, programmatic launches), planes / wide:
+//   own result   4 rows    t = 31 13.7 / 11.2, 37 14.3 / 14.6         6 rows    48 15.9 / 12.7, 55 16.2 / 17.0
+//                8 rows    t = 55 17.0 / 17.2 (K = 4096) and 17.9 / 17.4 (K = 8192), 96 21.0 / 23.1
+//                9 rows    t = 55 19.2 / 17.2, 96 22.7 / 23.1         12 rows   96 24.2 / 23.3, 138 28.9 / 28.9
+//                16 rows   t = 138 30.6 / 29.3, 193 34.8 / 36.5       from 17 rows on always (t = 387 at 17: 67 / 65)
+//                (the planes step up at 9 rows, from 32 to 64 MMA columns: hence two lines)
+//   added into a stack, fp32 activations.  A block of the stack with this product on planes / wide:
+//                9 to 16 rows: the wide kernel's own loaders convert them and fall behind on large matrices, the earlier
+//                the fewer rows there are to gain from: 9 rows t = 47 72.5 / 72.1, 55 101.8 / 102.1, 58 59.5 / 61.4; 16
+//                rows t = 55 106.8 / 106.2, 58 63.3 / 64.4
+//                17 to 32 rows: both kernels read converted ones.  Behind silu(gate) * up the planes kernel is the dearer
+//                of the two conversions by some 2 us (t = 98 at 24 rows 97.2 / 92.2); plain at 24 rows t = 41
+//                60.4 / 60.0, 64 75.7 / 75.0, 69 139.3 / 142.8
+static bool wide_is_faster(long long M, long long N, long long K, int x_kind, bool atomic, int num_sms) {
     const long long per_sm = (N + 255) / 256 * (K / 32) / num_sms;
-    if (fused) return M > 32 || (M > 16 ? per_sm <= 107 : M > 8 && per_sm <= 60);
-    return M > 16 || (M >= 4 && per_sm <= 15 * M - 28);
+    if (x_kind == DMM_X_F16 && !atomic) {
+        if (M <= 8) return M >= 4 && per_sm <= (M == 4 ? 32 : 5 * M + 19);
+        return M > 16 || per_sm <= 11 * M - 9;
+    }
+    if (M <= 8) return false;
+    if (M <= 16) return per_sm <= (x_kind == DMM_X_F16 ? 60 : 40 + M);
+    return M > 32 || per_sm <= (x_kind == DMM_X_F32 ? 64 : 107);
 }
 
 static size_t workspace_need(long long M, long long K, int num_sms) {
@@ -291,7 +304,7 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
     void *ws = nullptr;
     rc = resolve_workspace(d, M, K, workspace, workspace_bytes, stream, &ws);
     if (rc) return rc;
-    if (may_go_wide && wide_is_faster(M, N, K, x_kind != DMM_X_F16 || (flags & DMM_FLAG_ATOMIC) != 0, d->num_sms))
+    if (may_go_wide && wide_is_faster(M, N, K, x_kind, (flags & DMM_FLAG_ATOMIC) != 0, d->num_sms))
         return run_wide(x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K, sign_convention, flags, workspace,
                         workspace_bytes, stream, zero_ptr, zero_count, fast_layout);
     const long long step = f8 ? 32 : 64;
