@@ -297,7 +297,7 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
                     const void *cb16, float scale, float *out, long long M, long long N, long long K,
                     int sign_convention, unsigned flags, void *workspace, size_t workspace_bytes, cudaStream_t stream,
                     float *zero_ptr = nullptr, long long zero_count = 0, const TpArgs *tp = nullptr, bool fast_layout = false,
-                    bool may_go_wide = false) {
+                    bool may_go_wide = false, int handover = 0) {
     DeviceState *d = nullptr;
     int rc = current_device_state(&d);
     if (rc) return rc;
@@ -370,7 +370,7 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
         }
         // 17 to 32 batch rows (128 MMA columns) run on the kernel of dmm_tc.cuh, measured faster there;
         // everything else on the kernel of dmm_umma.cuh
-        rc = (f8 && p.M > 16 && !fast_layout) ? launch_tc_wide(p, d->num_sms, pdl, stream) : launch_umma(f8, p, d->num_sms, pdl, stream);
+        rc = (f8 && p.M > 16 && !fast_layout) ? launch_tc_wide(p, d->num_sms, pdl, stream) : launch_umma(f8, p, d->num_sms, pdl, stream, handover);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (rc) return rc;
     }
@@ -449,26 +449,11 @@ static int noalloc_scratch(void **out) {
     return 0;
 }
 
-}  // namespace dmm
-
-using namespace dmm;
-
-extern "C" {
-
-int dmm_i8(const int8_t *x, const int16_t *codes, const int64_t *cb64, int32_t *out, int64_t M, int64_t N, int64_t K,
-           int sign_convention, int layout, unsigned flags, void *workspace, size_t workspace_bytes, void *stream) {
-    int rc = check_common(x, codes, cb64, out, M, N, K, sign_convention, layout);
-    if (rc) return rc;
-    // the tcgen05 kernel streams either layout as it lies in memory
-    if (layout == DMM_LAYOUT_FAST && N % 32 != 0) return DMM_ERR_SHAPE;
-    return run_umma_i8(x, codes, cb64, out, M, N, K, sign_convention, flags, workspace, workspace_bytes,
-                       static_cast<cudaStream_t>(stream), layout == DMM_LAYOUT_FAST);
-}
-
-int dmm_f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, const int16_t *codes, const void *cb16,
-                  float scale, float *out, int64_t M, int64_t N, int64_t K, int sign_convention, int layout, int path,
-                  unsigned flags, float *zero_ptr, int64_t zero_count, void *workspace, size_t workspace_bytes,
-                  void *stream) {
+// dmm_f16_fused; handover as in launch_umma
+static int f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, const int16_t *codes, const void *cb16,
+                     float scale, float *out, int64_t M, int64_t N, int64_t K, int sign_convention, int layout, int path,
+                     unsigned flags, float *zero_ptr, int64_t zero_count, void *workspace, size_t workspace_bytes,
+                     void *stream, int handover) {
     int rc = check_common(x, codes, cb16, out, M, N, K, sign_convention, layout);
     if (rc) return rc;
     if (path != DMM_PATH_AUTO && path != DMM_PATH_GEMV && path != DMM_PATH_TCGEN05 && path != DMM_PATH_TCGEN05_F8)
@@ -500,11 +485,35 @@ int dmm_f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, const 
     if (path == DMM_PATH_TCGEN05 || path == DMM_PATH_TCGEN05_F8)
         return run_umma(path == DMM_PATH_TCGEN05_F8, x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K,
                         sign_convention, flags, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), zero_ptr,
-                        zero_count, nullptr, fast_native, any_path && path == DMM_PATH_TCGEN05_F8);
+                        zero_count, nullptr, fast_native, any_path && path == DMM_PATH_TCGEN05_F8, handover);
     if (x_ld != K) return DMM_ERR_UNSUPPORTED;
     // the streaming kernel accumulates quarter units: fold the 1/4 into the scale
     return run_stream(1, x, codes, cb16, 1, 0.25f * scale, out, M, N, K, sign_convention, flags, workspace,
                       workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace dmm
+
+using namespace dmm;
+
+extern "C" {
+
+int dmm_i8(const int8_t *x, const int16_t *codes, const int64_t *cb64, int32_t *out, int64_t M, int64_t N, int64_t K,
+           int sign_convention, int layout, unsigned flags, void *workspace, size_t workspace_bytes, void *stream) {
+    int rc = check_common(x, codes, cb64, out, M, N, K, sign_convention, layout);
+    if (rc) return rc;
+    // the tcgen05 kernel streams either layout as it lies in memory
+    if (layout == DMM_LAYOUT_FAST && N % 32 != 0) return DMM_ERR_SHAPE;
+    return run_umma_i8(x, codes, cb64, out, M, N, K, sign_convention, flags, workspace, workspace_bytes,
+                       static_cast<cudaStream_t>(stream), layout == DMM_LAYOUT_FAST);
+}
+
+int dmm_f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, const int16_t *codes, const void *cb16,
+                  float scale, float *out, int64_t M, int64_t N, int64_t K, int sign_convention, int layout, int path,
+                  unsigned flags, float *zero_ptr, int64_t zero_count, void *workspace, size_t workspace_bytes,
+                  void *stream) {
+    return f16_fused(x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K, sign_convention, layout, path, flags, zero_ptr,
+                     zero_count, workspace, workspace_bytes, stream, 0);
 }
 
 int dmm_f16(const void *x, const int16_t *codes, const void *cb16, float scale, float *out, int64_t M, int64_t N,
@@ -874,6 +883,14 @@ int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_con
                      void *stream) {
     if (!ops) return DMM_ERR_NULL;
     if (n_ops < 1) return DMM_ERR_ARG;
+    // The products share one choice of the hand-over, because two kernels in turn cost more than the better one for each
+    // gains: a block of a stack of width 3072 takes 24.3 us so, and 23.3 or 24.1 with either kernel alone.
+    HandoverSize size;
+    DeviceState *d = nullptr;
+    if (current_device_state(&d) == 0)  // (else the first op says why not)
+        for (int i = 0; i < n_ops; ++i)
+            if (ops[i].N >= 16 && ops[i].N <= (1ll << 24) && ops[i].K >= 32 && ops[i].K <= (1ll << 17))  // (others will be refused)
+                size.add(ops[i].N, ops[i].K, d->num_sms);
     for (int i = 0; i < n_ops; ++i) {
         const dmm_fused_op &op = ops[i];
         int rc = 0;
@@ -883,9 +900,9 @@ int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_con
             t_next_hint = NextHint();  // that op's own call will refuse it; this one is launched all the same
         }
         if (rc == 0)
-            rc = dmm_f16_fused(op.x, op.x_kind, op.x_ld, op.x_gap, op.codes, op.cb16, op.scale, op.out, M, op.N, op.K,
-                               sign_convention, DMM_LAYOUT_TILE, DMM_PATH_AUTO, flags, op.zero_ptr, op.zero_count, workspace,
-                               workspace_bytes, stream);
+            rc = f16_fused(op.x, op.x_kind, op.x_ld, op.x_gap, op.codes, op.cb16, op.scale, op.out, M, op.N, op.K, sign_convention,
+                           DMM_LAYOUT_TILE, DMM_PATH_AUTO, flags, op.zero_ptr, op.zero_count, workspace, workspace_bytes, stream,
+                           size.k_tiles());
         if (rc) {
             t_next_hint = NextHint();
             return rc;

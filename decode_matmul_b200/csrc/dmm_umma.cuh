@@ -20,7 +20,7 @@
 //   PolF16  fp16 family, fp16 operands (DMM_PATH_TCGEN05): weights as fp16 integers q (byte ->
 //           half by magic number), activations as fp16, kind::f16, K = 16.  A cross-check.
 //   PolF8Fast / PolI8Fast: the same over codes in the layout of fast_decode_matmul_cuda.
-//   PolF8Long: PolF8 with one hand-over per four k-tiles (16 and 64 columns).
+//   PolF8Long: PolF8 with one hand-over per four k-tiles (64 columns, and large matrices at 16).
 // Template flags: kChain (several dependent products in one cooperative launch, the CTAs stay
 // resident), kTp (tensor-parallel forms: epilogue that adds into every rank's buffer, producer
 // and consumer of the slots form) and kSplit (four TMA producer warps, batch 1 and 2).
@@ -208,9 +208,9 @@ struct PolF8 {
 };
 // The same with one hand-over per four k-tiles instead of two, in one group buffer of twice the size: half the waits,
 // fences, arrivals and commits per tile, and the decoders, which are short of issue slots, gain it.  A block of the
-// 70B stack at batch 1 70.5 us (72.5 with PolF8), at 2 77.9 (79.8), at 16 105.5 (112.5).  Not for the
-// 32-column build, whose single accumulator set has nothing to hide the longer hand-over at the end of a segment
-// behind (batch 4: 90.7 against 85.3), nor for int8 (4096 x 4096: 8.0 against 7.6).
+// 70B stack at batch 1 71.6 us (73.6 with PolF8), at 2 78.4 (80.8), at 16 105.6 (112.7).  For batch 1 and 2 only where the
+// segments are long (HandoverSize).  Not for the 32-column build, whose single accumulator set has nothing to hide the longer
+// hand-over at the end of a segment behind (batch 4: 90.7 against 85.3), nor for int8 (4096 x 4096: 8.0 against 7.6).
 struct PolF8Long : PolF8 {
     static constexpr int kG = 4;
     static constexpr int kNA = 1;
@@ -1807,8 +1807,25 @@ inline int launch_umma_i8(const UmmaParams &p, int num_sms, bool pdl, cudaStream
     return launch_umma_one<PolI8, 32>(p, num_sms, pdl, stream);
 }
 
-// f8 != 0: PolF8 (needs M <= 32); else PolF16 with M <= 64.
-inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cudaStream_t stream) {
+// Batch 1 and 2: four k-tiles per hand-over instead of two (PolF8Long) from 28 tiles per segment on.  The longer hand-over
+// gains with every tile and loses some 0.2 us at the end of each segment, where nothing is left to decode beside the MMAs
+// of the last one.  A CTA has about 1 + super-tiles / SMs segments.  PolF8 / PolF8Long in us, batch 1, added into a stack, and
+// tiles per segment: 57344 x 512 6.81 / 7.32 (10), 4096 x 4096 5.17 / 5.45 (13), 40960 x 1024 7.58 / 7.88 (17), 57344 x 1024 8.64 / 8.88
+// (19), 16384 x 2048 6.57 / 6.75 (19), 6144 x 6144 6.70 / 6.82 (27), 11008 x 4096 7.58 / 7.56 (29; a result of its own 10.93 / 10.82),
+// 57344 x 2048 13.14 / 13.13 (39), 8192 x 8192 9.11 / 9.00 (45), 28672 x 8192 20.6 / 20.1 (110).
+struct HandoverSize {
+    long long tiles = 0, segments = 0;  // of all CTAs
+    void add(long long N, long long K, int num_sms) {
+        const long long sst = (N + 255) / 256;
+        tiles += sst * (K / 32);
+        segments += sst + num_sms;
+    }
+    int k_tiles() const { return tiles >= 28 * segments ? 4 : 2; }
+};
+
+// f8 != 0: PolF8 (needs M <= 32); else PolF16 with M <= 64.  handover: k-tiles per hand-over at batch 1 and 2, 0 for what
+// suits this product alone.
+inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cudaStream_t stream, int handover = 0) {
     if (f8 && p.fast_layout) {
         if (p.M <= 8) return launch_umma_one<PolF8Fast, 32>(p, num_sms, pdl, stream);
         if (p.M <= 16) return launch_umma_one<PolF8Fast, 64>(p, num_sms, pdl, stream);
@@ -1818,7 +1835,15 @@ inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cuda
         // up to two batch rows all four planes fit one 8-row core matrix: 16 MMA columns instead of 32 halve
         // what the tensor core reads from shared memory per MMA (the build with four TMA producers).  For 3
         // and 4 rows (two core matrices of the dense planes) it measured 1-2 % faster but cost batch 2 3 %.
-        if (p.M <= 2) return launch_umma_one<PolF8Long, 16>(p, num_sms, pdl, stream);
+        if (p.M <= 2) {
+            if (handover == 0) {
+                HandoverSize alone;
+                alone.add(p.N, p.K, num_sms);
+                handover = alone.k_tiles();
+            }
+            if (handover == 4) return launch_umma_one<PolF8Long, 16>(p, num_sms, pdl, stream);
+            return launch_umma_one<PolF8, 16>(p, num_sms, pdl, stream);
+        }
         if (p.M <= 8) return launch_umma_one<PolF8, 32>(p, num_sms, pdl, stream);
         if (p.M <= 16) return launch_umma_one<PolF8Long, 64>(p, num_sms, pdl, stream);
         return launch_umma_one<PolF8, 128>(p, num_sms, pdl, stream);

@@ -49,3 +49,23 @@ def test_lines(M, x_kind, limit):
                                                (33, _lib.X_F32, 220, False)])
 def test_beyond_the_lines(M, x_kind, t, planes):
     assert _on_planes(M, t, x_kind) == planes
+
+
+# batch 1 and 2: two k-tiles per hand-over where segments are short, four on the others (HandoverSize: 28 tiles per
+# segment; with 148 SMs the line lies between 2496 and 2528 at 82 super-tiles); numbers of k-tiles that neither divides
+@pytest.mark.parametrize("N,K", [(16, 32), (272, 2048), (20992, 2496), (20992, 2528), (20976, 2656), (57344, 1056), (57344, 1600),
+                                 (4112, 8256), (4112, 10528)])
+@pytest.mark.parametrize("M", [1, 2])
+def test_hand_over_of_two_and_of_four(M, N, K):
+    gen = torch.Generator(device="cuda").manual_seed(N + K)
+    codes = torch.randint(-32768, 32768, (N, K // 8), dtype=torch.int16, device="cuda", generator=gen)
+    cb = torch.from_numpy(o.synthetic_codebook(42)).cuda()
+    x = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
+    w = dmm.decode_weights(codes, cb)
+    want = torch.cat([x.double() @ part.double().T for part in w.split(16384)], dim=1)
+    base = torch.randn((M, N), device="cuda", generator=gen)
+    # exact products, sums off by the truncation of the tensor core: 7e-7 to 9e-7 at any length
+    for out, kw, ref in ((None, {}, want), (base.clone(), dict(accumulate=True, atomic=True), want + base)):
+        y = dmm.decode_matmul_fp16(x, codes, cb, 1.0, out, **kw).double()
+        assert float((y - ref).norm() / ref.norm()) <= 2e-6
+    assert dmm.status() == 0
