@@ -138,17 +138,122 @@ def test_wide_rows_of_a_larger_buffer():
         assert _rel(out.cpu().numpy(), want) <= REL
 
 
+def _device_case(M, N, K, x_positive=False, w_positive=False):
+    """Inputs made on the GPU, for sizes that are too large for the oracle: x, tiled codes, table, and the product in 64 bits
+    from decode_weights, which equals the oracle's decode bit for bit (test_gpu_decode_weights.py)."""
+    gen = torch.Generator(device="cuda").manual_seed(M + N + K)
+    cb = _dev(o.cb64_to_cb16(np.ascontiguousarray(o.build_codebook_abs())))
+    if w_positive:
+        table = o.decode_table(np.ascontiguousarray(o.build_codebook_abs()), o.SIGN_SLOW).reshape(65536, 8)
+        words = _dev(np.arange(65536, dtype=np.uint16).view(np.int16)[(table > 0).all(1)])
+        codes = words[torch.randint(0, len(words), (N, K // 8), device="cuda", generator=gen)]
+    else:
+        codes = torch.randint(-32768, 32768, (N, K // 8), dtype=torch.int16, device="cuda", generator=gen)
+    x = torch.randn((M, K), device="cuda", generator=gen).to(torch.float16)
+    x = x.abs() if x_positive else x
+    want = torch.empty((M, N), dtype=torch.float64, device="cuda")
+    for n0 in range(0, N, 8192):
+        rows = dmm.decode_weights(dmm.transpose_tile(codes[n0:n0 + 8192]), cb).double()
+        want[:, n0:n0 + 8192] = x.double() @ rows.T
+    return x, dmm.transpose_tile(codes), cb, want
+
+
+def _off(y, want):
+    return float((y.double() - want).norm() / want.norm())
+
+
+def _sms():
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+# One tile more than there are CTAs and one less than half as many again: every CTA has a whole tile of 25 units (three
+# chains in each build: 32, 64 and 128 columns, the last one also as three column tiles of 112), and some a part of a split
+# one behind it, which ends with a quarter of a unit.  The rows end in the last strip but one of a super-tile.
+@pytest.mark.parametrize("rest", [1, 68])
+@pytest.mark.parametrize("M", [20, 64, 128, 333])
+def test_whole_tiles_of_several_chains_and_split_ones(M, rest):
+    K = 3104
+    N = 256 * ((_sms() + rest + 2) // (3 if M == 333 else 1)) - 16
+    x, tiled, cb, want = _device_case(M, N, K)
+    base = torch.randn((M, N), device="cuda")
+    first = dmm.decode_matmul_fp16(x, tiled, cb)
+    assert _off(first, want) <= 1e-6  # see test_error_of_long_reductions
+    assert torch.equal(first, dmm.decode_matmul_fp16(x, tiled, cb)), "the summation order must be fixed"
+    for atomic in (False, True):
+        y = dmm.decode_matmul_fp16(x, tiled, cb, 1.0, base.clone(), accumulate=True, atomic=atomic)
+        assert _off(y, want + base) <= 1e-6
+
+
+# The tensor core truncates when it adds to its accumulator.  Cut into chains of at most 88 MMAs the sums of random terms
+# were off by at most 6.2e-7, whatever the length; not cut, by 2.6e-5 at this one.  Terms of one sign are the
+# worst case, since the truncations then add up: each takes at most 2^-23 of a sum that grows evenly, so at most
+# 88 * 2^-23 / 2 = 5.2e-6 over a chain and about a quarter of that for uniform mantissas and remainders; measured 1.3e-6.
+@pytest.mark.parametrize("one_signed", [False, True])
+@pytest.mark.parametrize("M,tiles", [(16, 1), (17, 148), (64, 1), (64, 148), (100, 148), (128, 148), (333, 50)])
+def test_error_of_long_reductions(M, tiles, one_signed):
+    x, tiled, cb, want = _device_case(M, 256 * tiles, 28672, one_signed, one_signed)
+    assert _off(dmm.decode_matmul_fp16(x, tiled, cb), want) <= (2e-6 if one_signed else 1e-6)
+
+
 def test_small_workspace_leaves_the_tiles_whole():
-    """A caller's workspace that only fits the narrower kernels is accepted, as is one of the full size."""
-    M, N, K = 333, 512, 1024
-    x, codes, cb16 = _case(M, N, K, 6)
-    want = _want(x, codes, cb16)
+    """A caller's workspace that only fits the narrower kernels is accepted and not written past its end; the tiles that are
+    split in one of the full size (whose sums then come out in another order) are computed whole."""
+    M, N, K = 128, 256 * (_sms() + 68) - 16, 3104
+    x, tiled, cb, want = _device_case(M, N, K)
     full = dmm.workspace_bytes(M, N, K)
-    for size in (full, full - 256, dmm.workspace_bytes(64, N, K) if dmm.workspace_bytes(64, N, K) < full else full):
-        ws = torch.zeros((size,), dtype=torch.uint8, device="cuda")
+    small = dmm.workspace_bytes(64, N, K)
+    assert small < full - 256
+    got = []
+    for size in (full, full - 256, small):
+        room = torch.zeros((full + (64 << 20),), dtype=torch.uint8, device="cuda")
+        room[size:] = 0x5A
         out = torch.empty((M, N), device="cuda")
-        dmm.decode_matmul_fused(_dev(x), _dev(o.tile_pack(codes)), _dev(cb16), 1.0, out, x_kind=_lib.X_F16, workspace=ws)
-        assert _rel(out.cpu().numpy(), want) <= REL
+        dmm.decode_matmul_fused(x, tiled, cb, 1.0, out, x_kind=_lib.X_F16, workspace=room[:size])
+        assert _off(out, want) <= 1e-6
+        assert bool((room[size:] == 0x5A).all())
+        got.append(out)
+    assert torch.equal(got[1], got[2]) and not torch.equal(got[0], got[1])
+
+
+# the kernel's own loaders (up to 16 rows) and half_kernel in front of it, over the layout of fast_decode_matmul_cuda, which only
+# the C entry combines with fp32 activations
+@pytest.mark.parametrize("M", [9, 16, 24])
+@pytest.mark.parametrize("silu", [False, True])
+def test_fast_layout_with_fp32_inputs(M, silu):
+    N, K = 544, 1056
+    x, codes, cb16 = _case(M, N, K, 11)
+    rng = np.random.default_rng(12)
+    xf = rng.standard_normal((M, 2 * K if silu else K)).astype(np.float32)
+    xt = torch.from_numpy(xf)
+    half = (torch.nn.functional.silu(xt[:, :K]) * xt[:, K:] if silu else xt).to(torch.float16).numpy()
+    want = _want(half, codes, cb16, o.SIGN_FAST)
+    xd, packed, cb = _dev(xf), dmm.fast_pack(_dev(codes)), _dev(cb16)
+    base = np.random.default_rng(13).standard_normal((M, N)).astype(np.float32)
+    for flags in (0, _lib.FLAG_ACCUMULATE | _lib.FLAG_ATOMIC):
+        out = _dev(base)
+        rc = _lib.lib().dmm_f16_fused(xd.data_ptr(), _lib.X_F32_SILU_MUL if silu else _lib.X_F32, xd.shape[1], K if silu else 0,
+                                      packed.data_ptr(), cb.data_ptr(), 1.0, out.data_ptr(), M, N, K, _lib.SIGN_FAST,
+                                      _lib.LAYOUT_FAST, _lib.PATH_AUTO, flags, None, 0, None, 0,
+                                      torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        # (silu uses the fast exponential, see test_fp32_inputs_and_clearing)
+        assert _rel(out.cpu().numpy(), want + (base if flags else 0)) <= (1e-4 if silu else REL)
+
+
+@pytest.mark.parametrize("batch", [9, 16, 24])
+def test_fused_step_that_mixes_the_kernels(batch):
+    """A block wide enough for the planes: of its four products one (o, at 24 rows also down) or none runs on the wide kernel.
+    Same result as the step with separate conversions."""
+    from decode_matmul_b200.linear import LinearStack
+
+    cfg = dict(hidden=8192, kv_heads=8, head_dim=128, ffn=14336, layers=1)
+    stack = LinearStack(cfg, dmm.synthetic_codebook(42), "cuda", seed=6, scale=2.0 ** -10)
+    h0 = torch.randn(batch, 8192, device="cuda", generator=torch.Generator(device="cuda").manual_seed(batch))
+    h_fused = stack.step(h0.clone(), fused=True)
+    h_plain = stack.step(h0.clone(), fused=False, path=_lib.PATH_TCGEN05_F8)
+    # Of what the block adds.  Both steps round the same intermediate sums to halves; one that falls to the other side is
+    # off by 2^-11, and fewer than one in a hundred does: 2^-11 / 10.
+    assert float((h_fused - h_plain).norm() / (h_plain - h0).norm()) <= 5e-5
 
 
 @pytest.mark.parametrize("M", [32, 192])
