@@ -16,16 +16,25 @@
 //   tensor pipe      4 MMAs of NB / 2 cycles
 //   shared memory    96 table look-ups + 32 codes in and out + 1.5 NB
 //   integer ALU      9 operations per code and some 40 around them: 180 cycles
-// Measured 255 cycles per tile up to 32 columns (the decoders: latency of their waits and look-ups, ALU 70 % busy) and
-// 330 .. 350 at 128.  28672 x 8192: 34.6 us at 16 rows, 36.3 at 32 (the fp8 planes: 35.7, 48.1), 42.5 at 64, 62 at
-// 128; 2048 x 8192 x 28672 863 us (1.1 PFLOP/s; 3455 as passes of 32 rows).
+// Measured in the steady state (37888 x 8192 .. 32768, one tile per CTA, by the clock seen meanwhile): 270 cycles per tile
+// up to 32 columns (the decoders: latency of their waits and look-ups, ALU 70 % busy), 278 at 64, 330 at 112, 370 at 128, where
+// only one accumulator set fits and the tensor core waits while the sums are read.  28672 x 8192 with programmatic launches:
+// 36.9 us at 17 rows, 37.5 at 32 (the fp8 planes: 42.3, 49), 43 at 64, 62 at 128; 2048 x 8192 x 28672 746 us as a
+// single launch and 852 (1.13 PFLOP/s) back to back, when the power cap holds the clock at 1.4 GHz (3455 as passes of 32 rows).
+// 112- and 96-column tiles: 783 and 824 single, 886 and 939 back to back.
 //
 // Accuracy.  kind::f16 truncates when it adds to the accumulator: over a chain of n MMAs the sums shrink by a part
-// in 2^24 or so per MMA (measured against 64 bits: 4.2e-7 after 64, 9.7e-7 after 128, 2.6e-5 after 1792).
+// in 2^24 or so per MMA (measured against 64 bits, random terms: 4.2e-7 after 64, 9.7e-7 after 128, 2.6e-5 after 1792).
 // The fp8 planes stay at 7.5e-7 whatever the length.  So a chain is cut after at most kWChain units of 128 k (88
 // MMAs, 6.2e-7): the decoder warps add the accumulators to fp32 sums in registers (rounded to nearest) and the
-// next chain starts from zero.  That is why a column tile ends at 128: its sums are 64 registers per thread.
+// next chain starts from zero.  (Terms of one sign, activations and weights both, are the worst case: up to 1.3e-6, uncut 1.2e-4;
+// the planes 2e-7.)  That is why a column tile ends at 128: its sums are 64 registers per thread.
 // Up to 64 columns there are two accumulator sets, so the next chain starts while the last one is read.
+//
+// Registers.  The compiler allocates 96 per thread, whatever setmaxnreg adds later, and the sums do not leave enough: -Xptxas -v
+// shows 144 bytes of spill stores and 80 of loads at 64 columns, 348 and 176 at 128 (fast layout 360 and 152), none at 32.  ncu
+// counts some five local loads and as many stores per warp and half unit at 128 columns (from 28672 x 8192 against x 16384),
+// those of the chains and epilogues included.
 //
 // Work split.  A tile of output is (256 rows, NB columns); its reduction is cut into units of 128 k.  While
 // there are more tiles than CTAs every CTA computes whole tiles; the units of the tiles that remain are
@@ -760,6 +769,8 @@ inline int launch_wide(WideParams p, const void *x, int x_mode, long long x_ld, 
     if (rest > 0) {
         // How many CTAs share the remaining tiles: estimated cycles of the longest CTA.  A unit costs about
         // 640 + 10 nb, and a split tile a fix-up: its last CTA reads nb KiB per contributor at 64 bytes a cycle.
+        // (An estimate that ranks the splits well, not the rate: in the steady state a unit takes 1080 cycles up to 32
+        // columns and 1480 at 128.)
         long long parts = rest, best = 0;
         for (long long c = rest; can_split && c <= num_sms; c = c < num_sms && c + rest > num_sms ? num_sms : c + rest) {
             if (c > rest && c > rest * p.units) break;
