@@ -198,7 +198,7 @@ def run_reference(args):
 
 
 # ------------------------------------------------------------------------------------------
-# single-shape timing (BASELINE.json configs[1..3] and the batch-32 half of the metric)
+# single-shape timing (the Llama-2 7B and 70B shapes and the batch-32 half of the metric)
 # ------------------------------------------------------------------------------------------
 def time_shape(dmm, torch, family, batch, n, k, total_mb=700):
     """Median microseconds per call over 5 replays of a CUDA graph of back-to-back calls (programmatic
@@ -252,8 +252,8 @@ def time_shape(dmm, torch, family, batch, n, k, total_mb=700):
 
 
 def per_shape_table(dmm, torch, peaks):
-    """BASELINE.json configs[1] (Llama-2-7B shapes, batch 1), configs[2] (batch sweep on the 7B gate/up
-    and down shapes), configs[3] (Llama-2-70B shapes at batch 1 and 16) and the integer operator."""
+    """Llama-2-7B shapes at batch 1, a batch sweep on the 7B gate/up and down shapes, Llama-2-70B shapes at batch 1
+    and 16, and the integer operator."""
     rows = []
     for n, k in [(4096, 4096), (11008, 4096), (4096, 11008)]:
         rows.append(dict(time_shape(dmm, torch, "fp16", 1, n, k), config="configs[1]"))

@@ -54,8 +54,8 @@ static int current_device_state(DeviceState **out) {
 }
 
 // Size of the library's own workspace on first use: the tickets and behind them either the
-// partial tiles of the wide kernel (148 CTAs, 128 columns: 37 MiB) or stream-K partials at batch 64 (up to
-// 256 CTAs: 16 MiB) and the activation planes for K up to 2^17 (16 MiB).
+// partial tiles of the wide kernel (148 CTAs, 128 columns: 37 MiB) or stream-K partials at batch 64 (148 CTAs:
+// 18.5 MiB) and the activation planes for K up to 2^17 (16 MiB).
 constexpr size_t kDefaultWorkspace = size_t(42) << 20;
 
 // Counters of the split tiles, at the start of every workspace: one per CTA.  A split tile counts at the index of the

@@ -11,7 +11,7 @@ constexpr int kDecodeThreads = 1024;
 constexpr int kDecodeTiles = 4;  // k-tiles per work item of decode_kernel
 
 // Re-tiles codes from the layout of fast_decode_matmul_cuda -- flat uint32 [N/32][K/16][lane:32],
-// word = code(n = 32*nb + lane, j = 2*kp) | code(j = 2*kp + 1) << 16, the completion this build
+// word = code(n = 32*nb + lane, j = 2*kp) | code(j = 2*kp + 1) << 16, the completion this library
 // defines for the reference's lane-per-column reads (fast_decode_matmul_cuda.cu:106,110-113,130) --
 // into the tile layout [N/16][K/32][g:8][t:4][h:2] that every kernel of this library streams.
 // One warp per (32-row block, k-tile): 256 contiguous bytes in, 256 contiguous bytes out; lane l

@@ -31,7 +31,7 @@ def fast_pack(codes: torch.Tensor) -> torch.Tensor:
     [N/32][K/16][lane:32], word = code(n = 32*nb + lane, j = 2*kp) | code(j = 2*kp + 1) << 16.
     The reference's fast kernel reads one such word per lane, a warp covering 32 consecutive
     output columns (fast_decode_matmul_cuda.cu:106,110-113,130); its k addressing is not
-    self-consistent, so this build defines the completion.  Shape stays [N, K/8]."""
+    self-consistent, so this library defines the completion.  Shape stays [N, K/8]."""
     n, k8 = codes.shape
     if n % 32 or k8 % 4:
         raise RuntimeError("fast_pack: need N % 32 == 0 and K % 32 == 0")

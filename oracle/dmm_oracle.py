@@ -185,7 +185,7 @@ def tile_unpack(tiled: np.ndarray) -> np.ndarray:
 
 
 def fast_pack(codes: np.ndarray) -> np.ndarray:
-    """logical [N, K/8] -> the layout this build defines for ``fast_decode_matmul_cuda``.
+    """logical [N, K/8] -> the layout this library defines for ``fast_decode_matmul_cuda``.
 
     The reference's fast kernel reads one uint32 (two codes = 16 consecutive k of one
     output column) per lane, a warp covering 32 consecutive columns
