@@ -92,17 +92,18 @@ static size_t planes_offset(long long M, int num_sms) {
 //                the fewer rows there are to gain from: 9 rows t = 47 72.5 / 72.1, 55 101.8 / 102.1, 58 59.5 / 61.4; 16
 //                rows t = 55 106.8 / 106.2, 58 63.3 / 64.4
 //                17 to 32 rows: both kernels read converted ones.  Behind silu(gate) * up the planes kernel is the dearer
-//                of the two conversions by some 2 us (t = 98 at 24 rows 97.2 / 92.2); plain at 24 rows t = 41
-//                60.4 / 60.0, 64 75.7 / 75.0, 69 139.3 / 142.8
+//                of the two conversions by some 2 us (t = 98 at 24 rows 97.2 / 92.2).  Plain ones: the planes cost more
+//                per segment, the wide kernel per tile, so what counts is tiles per segment; at 24 rows 22016 x 4096 (47)
+//                60.3 / 59.5, 15360 x 5120 (46) 75.7 / 75.0, 8192 x 8192 (46) 141.2 / 139.3, 10240 x 8192 (54) 139.3 / 142.8
 static bool wide_is_faster(long long M, long long N, long long K, int x_kind, bool atomic, int num_sms) {
-    const long long per_sm = (N + 255) / 256 * (K / 32) / num_sms;
+    const long long sst = (N + 255) / 256, tiles = sst * (K / 32), per_sm = tiles / num_sms;
     if (x_kind == DMM_X_F16 && !atomic) {
         if (M <= 8) return M >= 4 && per_sm <= (M == 4 ? 32 : 5 * M + 19);
         return M > 16 || per_sm <= 11 * M - 9;
     }
     if (M <= 8) return false;
     if (M <= 16) return per_sm <= (x_kind == DMM_X_F16 ? 60 : 40 + M);
-    return M > 32 || per_sm <= (x_kind == DMM_X_F32 ? 64 : 107);
+    return M > 32 || (x_kind == DMM_X_F32 ? tiles <= 50 * (sst + num_sms) : per_sm <= 107);
 }
 
 static size_t workspace_need(long long M, long long K, int num_sms) {

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 def _on_planes(M, t, x_kind):
     """Whether a product of M rows with t tiles per SM runs on the plane kernels."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    N, K = 64 * sms, 128 * t  # sms / 4 super-tiles of 4 t k-tiles
+    N, K = 64 * sms, 128 * t  # sms / 4 super-tiles of 4 t k-tiles: 0.8 t tiles per segment
     assert sms % 4 == 0
     gen = torch.Generator(device="cuda").manual_seed(t)
     codes = torch.randint(-32768, 32768, (N, K // 8), dtype=torch.int16, device="cuda", generator=gen)
@@ -38,7 +38,7 @@ def _on_planes(M, t, x_kind):
 
 @pytest.mark.parametrize("M,x_kind,limit", [
     (4, _lib.X_F16, 32), (6, _lib.X_F16, 49), (8, _lib.X_F16, 59), (9, _lib.X_F16, 90), (12, _lib.X_F16, 123), (16, _lib.X_F16, 167),
-    (9, _lib.X_F32, 49), (16, _lib.X_F32, 56), (16, _lib.X_F32_SILU_MUL, 56), (17, _lib.X_F32, 64), (32, _lib.X_F32, 64),
+    (9, _lib.X_F32, 49), (16, _lib.X_F32, 56), (16, _lib.X_F32_SILU_MUL, 56), (17, _lib.X_F32, 62), (32, _lib.X_F32, 62),
     (17, _lib.X_F32_SILU_MUL, 107), (32, _lib.X_F32_SILU_MUL, 107)])
 def test_lines(M, x_kind, limit):
     assert not _on_planes(M, limit, x_kind)
