@@ -95,6 +95,8 @@ static size_t planes_offset(long long M, int num_sms) {
 //                of the two conversions by some 2 us (t = 98 at 24 rows 97.2 / 92.2).  Plain ones: the planes cost more
 //                per segment, the wide kernel per tile, so what counts is tiles per segment; at 24 rows 22016 x 4096 (47)
 //                60.3 / 59.5, 15360 x 5120 (46) 75.7 / 75.0, 8192 x 8192 (46) 141.2 / 139.3, 10240 x 8192 (54) 139.3 / 142.8
+//   added, fp16 activations (one product by itself): 9 rows t = 37 10.9 / 10.2, 55 12.7 / 12.8; 16 rows t = 55 13.3 / 13.1, 69
+//                14.6 / 15.2; 24 rows t = 96 22.0 / 19.3 (and 138 26.8 / 25.0: the line at 107 is that of the SiLU products)
 static bool wide_is_faster(long long M, long long N, long long K, int x_kind, bool atomic, int num_sms) {
     const long long sst = (N + 255) / 256, tiles = sst * (K / 32), per_sm = tiles / num_sms;
     if (x_kind == DMM_X_F16 && !atomic) {
@@ -102,7 +104,7 @@ static bool wide_is_faster(long long M, long long N, long long K, int x_kind, bo
         return M > 16 || per_sm <= 11 * M - 9;
     }
     if (M <= 8) return false;
-    if (M <= 16) return per_sm <= (x_kind == DMM_X_F16 ? 60 : 40 + M);
+    if (M <= 16) return per_sm <= 40 + M;
     return M > 32 || (x_kind == DMM_X_F32 ? tiles <= 50 * (sst + num_sms) : per_sm <= 107);
 }
 
