@@ -391,10 +391,12 @@ static int run_umma_i8(const void *x, const void *codes, const void *cb64, int32
     rc = resolve_workspace(d, M, K, workspace, workspace_bytes, stream, &ws);
     if (rc) return rc;
     // Integer sums do not depend on their order, so partial super-tiles are always added with
-    // atomics (no workspace round trip, no ticket); a plain product clears the output first.
+    // atomics (no workspace round trip, no ticket); a plain product clears the output first (not counted as a launch).
+    bool pdl = (flags & DMM_FLAG_PDL) != 0;
     if (!(flags & DMM_FLAG_ACCUMULATE)) {
-        const cudaError_t err = cudaMemsetAsync(out, 0, static_cast<size_t>(M) * static_cast<size_t>(N) * sizeof(int32_t), stream);
-        if (err != cudaSuccess) return err;
+        rc = launch_clear(out, M * N * static_cast<long long>(sizeof(int32_t)), d->num_sms, pdl, stream);
+        if (rc) return rc;
+        pdl = true;  // the first product may start beside the clearing
     }
     for (long long m0 = 0; m0 < M; m0 += 32) {
         UmmaParams p = {};
@@ -413,9 +415,10 @@ static int run_umma_i8(const void *x, const void *codes, const void *cb64, int32
         p.atomic_reduce = 1;
         p.sign_convention = sign_convention;
         p.fast_layout = fast_layout ? 1 : 0;
-        rc = launch_umma_i8(p, d->num_sms, (flags & DMM_FLAG_PDL) != 0, stream);
+        rc = launch_umma_i8(p, d->num_sms, pdl, stream);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (rc) return rc;
+        pdl = (flags & DMM_FLAG_PDL) != 0;
     }
     return 0;
 }
