@@ -289,7 +289,9 @@ template <class Pol, int NMMA>
 struct UmmaPlan {
     // accumulators per MMA tile = active issuers: one per decoder group while the TMEM holds them
     static constexpr int kNAcc = !Pol::kIsF8 ? 2 : (NMMA <= 32 ? 4 : (NMMA <= 64 ? 2 : 1));
-    static constexpr int kNA = Pol::kNA;
+    // int8 with 16 columns: the accumulators leave room for a third buffer per group, so that a decoder group seldom waits for
+    // the tensor core (16 x 8192 x 8192 16.5 -> 15.4 us; longer calls are bound by the look-ups: 8 x 28672 x 8192 26.9 both)
+    static constexpr int kNA = Pol::kIsInt && NMMA == 16 ? 3 : Pol::kNA;
     // issuer warps per accumulator: with fewer than four accumulators the two MMA tiles of a
     // group are issued by different warps (each accumulator still has exactly one issuer, so the
     // summation order stays fixed)
