@@ -282,7 +282,7 @@ static int run_wide(const void *x, int x_kind, long long x_ld, long long x_gap, 
 }
 
 // tcgen05 path: one launch per chunk of 64 batch columns (32 for the fp6/fp8 operand policy,
-// preceded by planes_kernel when the chunk has at least kPlanesMinBatch rows).
+// preceded by planes_kernel where planes_in_front says so).
 // Tensor-parallel extras of one call (dmm_f16_fused_tp).
 struct TpArgs {
     float *const *peer_out = nullptr;
@@ -300,7 +300,7 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
                     const void *cb16, float scale, float *out, long long M, long long N, long long K,
                     int sign_convention, unsigned flags, void *workspace, size_t workspace_bytes, cudaStream_t stream,
                     float *zero_ptr = nullptr, long long zero_count = 0, const TpArgs *tp = nullptr, bool fast_layout = false,
-                    bool may_go_wide = false, int handover = 0) {
+                    bool may_go_wide = false, const HandoverSize *group = nullptr) {
     DeviceState *d = nullptr;
     int rc = current_device_state(&d);
     if (rc) return rc;
@@ -316,7 +316,11 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
         UmmaParams p = {};
         p.x = reinterpret_cast<const uint8_t *>(x) + static_cast<size_t>(m0) * x_ld * (x_kind == DMM_X_F16 ? 2 : 4);
         p.M = M - m0 < step ? M - m0 : step;
-        if (f8 && p.M >= kPlanesMinBatch && !(tp != nullptr && tp->mode == 3)) {
+        // (a consumer of the slots form splits what it sums up itself; the other tensor-parallel products keep one line)
+        HandoverSize alone;
+        alone.add(N, K, d->num_sms);
+        if (f8 && (tp == nullptr ? planes_in_front(p.M, (group != nullptr ? group : &alone)->tiles_per_sm())
+                                 : tp->mode != 3 && p.M >= kPlanesMinBatch)) {
             // split the activations into E5M2 planes once, instead of once per CTA inside the kernel
             uint8_t *planes = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, d->num_sms);
             rc = launch_planes(p.x, x_kind, x_ld, x_gap, static_cast<int>(p.M), K, planes, pdl, stream);
@@ -373,7 +377,7 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
         }
         // 17 to 32 batch rows (128 MMA columns) run on the kernel of dmm_tc.cuh, measured faster there;
         // everything else on the kernel of dmm_umma.cuh
-        rc = (f8 && p.M > 16 && !fast_layout) ? launch_tc_wide(p, d->num_sms, pdl, stream) : launch_umma(f8, p, d->num_sms, pdl, stream, handover);
+        rc = (f8 && p.M > 16 && !fast_layout) ? launch_tc_wide(p, d->num_sms, pdl, stream) : launch_umma(f8, p, d->num_sms, pdl, stream, group);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (rc) return rc;
     }
@@ -455,11 +459,11 @@ static int noalloc_scratch(void **out) {
     return 0;
 }
 
-// dmm_f16_fused; handover as in launch_umma
+// dmm_f16_fused; group as in launch_umma
 static int f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, const int16_t *codes, const void *cb16,
                      float scale, float *out, int64_t M, int64_t N, int64_t K, int sign_convention, int layout, int path,
                      unsigned flags, float *zero_ptr, int64_t zero_count, void *workspace, size_t workspace_bytes,
-                     void *stream, int handover) {
+                     void *stream, const HandoverSize *group) {
     int rc = check_common(x, codes, cb16, out, M, N, K, sign_convention, layout);
     if (rc) return rc;
     if (path != DMM_PATH_AUTO && path != DMM_PATH_GEMV && path != DMM_PATH_TCGEN05 && path != DMM_PATH_TCGEN05_F8)
@@ -491,7 +495,7 @@ static int f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, con
     if (path == DMM_PATH_TCGEN05 || path == DMM_PATH_TCGEN05_F8)
         return run_umma(path == DMM_PATH_TCGEN05_F8, x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K,
                         sign_convention, flags, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), zero_ptr,
-                        zero_count, nullptr, fast_native, any_path && path == DMM_PATH_TCGEN05_F8, handover);
+                        zero_count, nullptr, fast_native, any_path && path == DMM_PATH_TCGEN05_F8, group);
     if (x_ld != K) return DMM_ERR_UNSUPPORTED;
     // the streaming kernel accumulates quarter units: fold the 1/4 into the scale
     return run_stream(1, x, codes, cb16, 1, 0.25f * scale, out, M, N, K, sign_convention, flags, workspace,
@@ -519,7 +523,7 @@ int dmm_f16_fused(const void *x, int x_kind, int64_t x_ld, int64_t x_gap, const 
                   unsigned flags, float *zero_ptr, int64_t zero_count, void *workspace, size_t workspace_bytes,
                   void *stream) {
     return f16_fused(x, x_kind, x_ld, x_gap, codes, cb16, scale, out, M, N, K, sign_convention, layout, path, flags, zero_ptr,
-                     zero_count, workspace, workspace_bytes, stream, 0);
+                     zero_count, workspace, workspace_bytes, stream, nullptr);
 }
 
 int dmm_f16(const void *x, const int16_t *codes, const void *cb16, float scale, float *out, int64_t M, int64_t N,
@@ -889,8 +893,9 @@ int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_con
                      void *stream) {
     if (!ops) return DMM_ERR_NULL;
     if (n_ops < 1) return DMM_ERR_ARG;
-    // The products share one choice of the hand-over, because two kernels in turn cost more than the better one for each
-    // gains: a block of a stack of width 3072 takes 24.3 us so, and 23.3 or 24.1 with either kernel alone.
+    // The products share one choice of the hand-over and of who splits the activations, because two kernels in turn cost more than
+    // the better one for each gains: a block of a stack of width 3072 takes 24.3 us so, and 23.3 or 24.1 with either kernel
+    // alone; one of width 5120 at 6 rows 50.7, and 49.5 with planes or 48.3 without.
     HandoverSize size;
     DeviceState *d = nullptr;
     if (current_device_state(&d) == 0)  // (else the first op says why not)
@@ -908,7 +913,7 @@ int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_con
         if (rc == 0)
             rc = f16_fused(op.x, op.x_kind, op.x_ld, op.x_gap, op.codes, op.cb16, op.scale, op.out, M, op.N, op.K, sign_convention,
                            DMM_LAYOUT_TILE, DMM_PATH_AUTO, flags, op.zero_ptr, op.zero_count, workspace, workspace_bytes, stream,
-                           size.k_tiles());
+                           size.sms > 0 ? &size : nullptr);
         if (rc) {
             t_next_hint = NextHint();
             return rc;

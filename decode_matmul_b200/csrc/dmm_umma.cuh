@@ -13,8 +13,8 @@
 //           the MMA n dimension (N = 16 / 32 / 64 / 128 columns for up to 2 / 8 / 16 / 32 batch
 //           rows; up to 2 rows the densely packed planes fit one 8-row core matrix), so
 //           one MMA per k-tile does all of them and the epilogue adds the four column groups.
-//           Up to 3 batch rows the loader warps split the activations themselves; from 4 rows
-//           on planes_kernel splits them once per call and the loaders only issue bulk copies.
+//           Up to 3 batch rows, and up to 8 on smaller matrices, the loader warps split the activations
+//           themselves; else planes_kernel splits them once per call and the loaders only issue bulk copies.
 //   PolI8   integer family (the reference's operator).  Weights as two's-complement bytes,
 //           int8 activations as they are, kind::i8 into int32 accumulators, N = 16 / 32.
 //   PolF16  fp16 family, fp16 operands (DMM_PATH_TCGEN05): weights as fp16 integers q (byte ->
@@ -55,6 +55,7 @@
 
 #include <atomic>
 #include <functional>
+#include <type_traits>
 #include <unordered_map>
 #include "dmm_common.cuh"
 #include "dmm_launch.h"
@@ -696,7 +697,10 @@ __global__ void __launch_bounds__(128) planes_kernel(const void *x, int x_mode, 
 // kTp == true adds the tensor-parallel pieces (adds into every rank's buffer, residual move).
 // kSplit == true is the instantiation with four TMA producer warps (28 warps; the register budget per
 // thread is smaller, which only the 32-column fp16-family kernel tolerates without a slow-down).
-template <class Pol, int NMMA, bool kChain, bool kTp = false, bool kSplit = false>
+// kPlanes == true: the activations come as planes that planes_kernel has split (from 9 batch rows on always); false: the loaders
+// split them (PolI8, PolF16: load them).  Two instantiations, because the decoders pay for the registers of whatever the loaders
+// carry: with both in one kernel the planes of a 4096-wide stack at batch 4 took 44.8 us per block instead of 41.7.
+template <class Pol, int NMMA, bool kChain, bool kTp = false, bool kSplit = false, bool kPlanes = false>
 __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps - 1) * 32, 1) umma_kernel(const __grid_constant__ UmmaChainT<kChain ? kMaxOps : 1> ch) {
     using Plan = UmmaPlan<Pol, NMMA>;
     constexpr int C = Pol::kC, G = Pol::kG, NA = Plan::kNA, RING = Pol::kRing, NACC = Plan::kNAcc, NB = Plan::kNB;
@@ -765,7 +769,7 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
             uint32_t count = 1;                                                // TMA, tcgen05.commit
             if (bt >= Plan::kBarEmpty && bt < Plan::kBarFull) count = 4;
             if (bt >= Plan::kBarFull && bt < Plan::kBarFree) count = Pol::kIsF8 ? 4 : 5;  // decoder warps (+ loader)
-            if (bt >= Plan::kBarXReady && bt < Plan::kBarXFree) count = p0.x_planes != nullptr ? 1 : kULoadWarps / kULoadTeams;
+            if (bt >= Plan::kBarXReady && bt < Plan::kBarXFree) count = kPlanes ? 1 : kULoadWarps / kULoadTeams;
             if (bt >= Plan::kBarFree && bt < Plan::kBarXReady) count = TP;  // tcgen05.commit of every issuer of the slot
             if (bt >= Plan::kBarXFree && bt < Plan::kBarDReady) count = NACC * TP;
             if (bt >= Plan::kBarDReady && bt < Plan::kBarDFree) count = NACC * TP;
@@ -1445,7 +1449,7 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
             const int nep = ntiles <= 0 ? 0 : (ntiles <= E0 ? 1 : 1 + (ntiles - E0 + E - 1) / E);
             // two teams of loader warps fill alternate epochs, so that the global-memory latency
             // of one epoch overlaps the plane split of the other
-            if (p.x_planes != nullptr && wl == 0 && lane == 0) {
+            if (kPlanes && wl == 0 && lane == 0) {
                 // The planes were split once by planes_kernel: an epoch is one bulk copy per
                 // contiguous run of k-tiles (two when the CTA's tile sequence wraps to the next
                 // super-tile inside the epoch).
@@ -1477,7 +1481,7 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
             const int lt = (wl / kULoadTeams) * 32 + lane;
             constexpr int LT = kULoadWarps / kULoadTeams * 32;
             // (team by the epoch number over all ops, so that the teams keep alternating across ops)
-            for (int e = ((wl % kULoadTeams) - eg_base) & (kULoadTeams - 1); p.x_planes == nullptr && e < nep; e += kULoadTeams) {
+            for (int e = ((wl % kULoadTeams) - eg_base) & (kULoadTeams - 1); !kPlanes && e < nep; e += kULoadTeams) {
                 const int eg = eg_base + e;
                 if (eg >= Plan::kEpochs)
                     mbar_wait(bar(Plan::kBarXFree + eg % Plan::kEpochs), static_cast<uint32_t>(((eg / Plan::kEpochs) - 1) & 1), flags);
@@ -1509,36 +1513,89 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
                         for (int u = 0; u < U; ++u)
                             if (dst[u] != 0) sts128(dst[u], val[u]);
                     }
-                } else
-                for (int pbase = 0; pbase < npieces; pbase += LT * U) {
-                    uint32_t h[U][4];
-                    uint32_t dst[U];
+                } else {
+                    // Where a piece lies: the division by the pieces per tile as a multiplication (exact: an epoch has less than
+                    // 2^16 / ppt pieces), the k-tile by stepping over the end of the row.
+                    const uint32_t ppt_inv = 65536u / static_cast<uint32_t>(ppt) + 1u;
+                    const int kt_lo = (i0 + t_lo) % KT;
+                    auto locate = [&](int pc, int &row, long long &k0) -> uint32_t {
+                        const int jl = static_cast<int>((static_cast<uint32_t>(pc) * ppt_inv) >> 16), rem = pc - jl * ppt, kc = rem & 3;
+                        row = rem >> 2;
+                        int kt = kt_lo + jl;
+                        while (kt >= KT) kt -= KT;
+                        k0 = 32ll * kt + 8 * kc;
+                        return ebuf + jl * tile_b + (kc >> 1) * (tile_b / 2) + row * 16 + (kc & 1) * 8;
+                    };
+                    auto store_planes = [&](uint32_t dst, uint32_t (&h)[4]) {
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int pc = pbase + u * LT + lt;
-                        dst[u] = 0;
-                        if (pc < npieces) {
-                            const int jl = pc / ppt, rem = pc - jl * ppt, row = rem >> 2, kc = rem & 3;
-                            const int gt = i0 + t_lo + jl;          // global tile index -> k-tile
-                            const int kt = gt - (gt / KT) * KT;
-                            const long long k0 = 32ll * kt + 8 * kc;
-                            dst[u] = ebuf + jl * tile_b + (kc >> 1) * (tile_b / 2) + row * 16 + (kc & 1) * 8;
-                            if (kTp && p.tp_mode == 3)
-                                load_piece_sum(reinterpret_cast<const float *>(p.x), p.h_out, tp_slots_now, p.tp_world, p.tp_count, p.x_ld,
-                                               row, k0, h[u]);
-                            else
-                                load_piece(p.x, p.x_mode, p.x_ld, p.x_gap, row, k0, h[u]);
+                        for (int pl = 0; pl < 4; ++pl) {
+                            const uint2 b8 = next_plane(h);
+                            sts64(dst + pl * (tile_b / 8), b8.x, b8.y);
                         }
-                    }
+                    };
+                    // UU pieces per thread: all loads first, at addresses that are always valid (with a branch around each piece they
+                    // went out one after the other, a round trip to L2 each), then the split of the pieces that are there.  Two
+                    // pieces: four spill.  A block of the 4096-wide stack at batch 1, 2 and 3 30.7, 33.2, 39.1 -> 29.5, 31.0, 36.2 us.
+                    auto stage = [&](auto uu, int pbase) {
+                        constexpr int UU = decltype(uu)::value;
+                        if (kTp && p.tp_mode == 3) {
+#pragma unroll 1
+                            for (int u = 0; u < UU; ++u) {
+                                const int pc = pbase + u * LT + lt;
+                                if (pc >= npieces) break;
+                                int row;
+                                long long k0;
+                                const uint32_t d = locate(pc, row, k0);
+                                uint32_t h[4];
+                                load_piece_sum(reinterpret_cast<const float *>(p.x), p.h_out, tp_slots_now, p.tp_world, p.tp_count, p.x_ld, row, k0, h);
+                                store_planes(d, h);
+                            }
+                            return;
+                        }
+                        uint32_t dst[UU];
+                        if (p.x_mode == kXHalf) {
+                            uint4 v[UU];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        if (dst[u] != 0) {
+                            for (int u = 0; u < UU; ++u) {
+                                const int pc = pbase + u * LT + lt;
+                                int row;
+                                long long k0;
+                                dst[u] = locate(pc < npieces ? pc : npieces - 1, row, k0);
+                                v[u] = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(p.x) + row * p.x_ld + k0));
+                            }
 #pragma unroll
-                            for (int pl = 0; pl < 4; ++pl) {
-                                const uint2 b8 = next_plane(h[u]);
-                                sts64(dst[u] + pl * (tile_b / 8), b8.x, b8.y);
+                            for (int u = 0; u < UU; ++u) {
+                                uint32_t h[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+                                if (pbase + u * LT + lt < npieces) store_planes(dst[u], h);
+                            }
+                            return;
+                        }
+                        float4 f[UU][2], g[UU][2];
+#pragma unroll
+                        for (int u = 0; u < UU; ++u) {
+                            const int pc = pbase + u * LT + lt;
+                            int row;
+                            long long k0;
+                            dst[u] = locate(pc < npieces ? pc : npieces - 1, row, k0);
+                            const float *xf = reinterpret_cast<const float *>(p.x) + row * p.x_ld + k0;
+                            f[u][0] = __ldcg(reinterpret_cast<const float4 *>(xf));
+                            f[u][1] = __ldcg(reinterpret_cast<const float4 *>(xf + 4));
+                            if (p.x_mode == kXSiluMul) {
+                                g[u][0] = __ldcg(reinterpret_cast<const float4 *>(xf + p.x_gap));
+                                g[u][1] = __ldcg(reinterpret_cast<const float4 *>(xf + p.x_gap + 4));
                             }
                         }
+#pragma unroll
+                        for (int u = 0; u < UU; ++u) {
+                            uint32_t h[4];
+                            pack_piece(p.x_mode, f[u], g[u], h);
+                            if (pbase + u * LT + lt < npieces) store_planes(dst[u], h);
+                        }
+                    };
+                    if (npieces <= LT) {
+                        stage(std::integral_constant<int, 1>{}, 0);
+                    } else {
+                        for (int pbase = 0; pbase < npieces; pbase += LT * 2) stage(std::integral_constant<int, 2>{}, pbase);
                     }
                 }
                 fence_async_smem();
@@ -1686,12 +1743,25 @@ inline int launch_umma_ops(const UmmaParams *ops, int n_ops, unsigned *sync, int
 template <class Pol, int NMMA, bool kChain>
 inline int launch_umma_ops(const UmmaParams *ops, int n_ops, unsigned *sync, int num_sms, bool pdl, cudaStream_t stream) {
     using Plan = UmmaPlan<Pol, NMMA>;
-    auto kernel = umma_kernel<Pol, NMMA, kChain, false>;
+    // planes: from 64 columns (9 batch rows) on always, with 16 columns (2 rows) and in chains never
+    constexpr bool only_planes = Pol::kIsF8 && !Pol::kIsInt && NMMA >= 64;
+    constexpr bool both = Pol::kIsF8 && !Pol::kIsInt && NMMA == 32 && !kChain;
+    const bool planes = only_planes || (both && ops[0].x_planes != nullptr);
+    if ((ops[0].x_planes != nullptr) != planes) return DMM_ERR_ARG;
+    auto kernel = umma_kernel<Pol, NMMA, kChain, false, false, only_planes>;
+    if constexpr (both) {
+        if (planes) kernel = umma_kernel<Pol, NMMA, kChain, false, false, true>;
+    }
     // four TMA producer warps up to two batch rows of the fp16 family (measured 1 % faster at batch 1), else one
     bool split = false;
     [[maybe_unused]] const bool tp_variant = ops[0].n_peers > 0 || ops[0].move_count > 0 || ops[0].tp_mode != 0;
     if constexpr (Pol::kIsF8 && !kChain && !Pol::kFast) {  // tensor-parallel epilogue: its own instantiation, nothing of it in the plain kernel
-        if (tp_variant) kernel = umma_kernel<Pol, NMMA, kChain, true>;
+        if (tp_variant) {
+            kernel = umma_kernel<Pol, NMMA, kChain, true, false, only_planes>;
+            if constexpr (both) {
+                if (planes) kernel = umma_kernel<Pol, NMMA, kChain, true, false, true>;
+            }
+        }
     }
     if constexpr (Pol::kIsF8 && !Pol::kIsInt && !kChain && NMMA == 16 && !Pol::kFast) {
         if (ops[0].M <= 2) {
@@ -1701,8 +1771,8 @@ inline int launch_umma_ops(const UmmaParams *ops, int n_ops, unsigned *sync, int
         }
     }
     // the shared-memory attribute is set once per kernel variant and device, not on every launch
-    static std::atomic<unsigned long long> attr_done[4];
-    const int variant = (tp_variant ? 1 : 0) | (split ? 2 : 0);
+    static std::atomic<unsigned long long> attr_done[8];
+    const int variant = (tp_variant ? 1 : 0) | (split ? 2 : 0) | (planes ? 4 : 0);
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;
@@ -1777,9 +1847,18 @@ inline int launch_umma_chain(const UmmaParams *ops, int n_ops, unsigned *sync, i
     return launch_umma_ops<PolF8, 32, true>(ops, n_ops, sync, num_sms, pdl, stream);
 }
 
-// From this batch size on the fp8-operand path splits the activations into planes with
-// planes_kernel before the matmul kernel instead of inside it.
+// Whether the activations of a chunk of M <= 32 rows are split into planes once, by a kernel in front of the product, or by
+// the product's own loaders in every CTA.  The kernel in front is one more dependent launch, 2 to 3 us; the loaders' split
+// costs nothing up to 3 rows and then more with every row and tile, hence a number of tiles per SM for each row count.  us per
+// block of a stack, planes / loaders, and its products' mean tiles per SM: 4 rows 41.2 / 35.8 (42), 49.0 / 44.4 (65), 86.8 / 84.4 (176);
+// 5 rows 41.7 / 36.8, 49.3 / 45.8, 87.5 / 88.9; 6 rows 41.9 / 37.7, 49.5 / 48.3, 86.2 / 95.4; 7 rows 42.3 / 38.4, 50.0 / 50.4,
+// 88.3 / 102.0; 8 rows 42.6 / 40.4, 50.4 / 51.5, 88.9 / 108.8.  One product by itself: 4 rows 28672 x 8192 (194) 27.1 / 26.7, 8
+// rows 29.4 / 32.5.  The lines lie where straight lines through these meet.
 constexpr long long kPlanesMinBatch = 4;
+inline bool planes_in_front(long long M, long long tiles_per_sm) {
+    constexpr int kMost[9] = {0, 0, 0, 0, 290, 144, 77, 63, 58};
+    return M > 8 || (M >= kPlanesMinBatch && tiles_per_sm > kMost[M]);
+}
 
 // Padded batch rows of the plane layout for a batch of M (<= 32) rows.
 inline int planes_rows(long long M) { return M <= 8 ? static_cast<int>(M) : (M <= 16 ? 16 : 32); }
@@ -1840,18 +1919,20 @@ inline int launch_umma_i8(const UmmaParams &p, int num_sms, bool pdl, cudaStream
 // (19), 16384 x 2048 6.57 / 6.75 (19), 6144 x 6144 6.70 / 6.82 (27), 11008 x 4096 7.58 / 7.56 (29; a result of its own 10.93 / 10.82),
 // 57344 x 2048 13.14 / 13.13 (39), 8192 x 8192 9.11 / 9.00 (45), 28672 x 8192 20.6 / 20.1 (110).
 struct HandoverSize {
-    long long tiles = 0, segments = 0;  // of all CTAs
+    long long tiles = 0, segments = 0, sms = 0;  // of all CTAs; SMs of all products
     void add(long long N, long long K, int num_sms) {
         const long long sst = (N + 255) / 256;
         tiles += sst * (K / 32);
         segments += sst + num_sms;
+        sms += num_sms;
     }
     int k_tiles() const { return tiles >= 28 * segments ? 4 : 2; }
+    long long tiles_per_sm() const { return tiles / sms; }
 };
 
-// f8 != 0: PolF8 (needs M <= 32); else PolF16 with M <= 64.  handover: k-tiles per hand-over at batch 1 and 2, 0 for what
-// suits this product alone.
-inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cudaStream_t stream, int handover = 0) {
+// f8 != 0: PolF8 (needs M <= 32); else PolF16 with M <= 64.  group: the products that share one choice of the hand-over, null for
+// this product alone.
+inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cudaStream_t stream, const HandoverSize *group = nullptr) {
     if (f8 && p.fast_layout) {
         if (p.M <= 8) return launch_umma_one<PolF8Fast, 32>(p, num_sms, pdl, stream);
         if (p.M <= 16) return launch_umma_one<PolF8Fast, 64>(p, num_sms, pdl, stream);
@@ -1862,12 +1943,9 @@ inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cuda
         // what the tensor core reads from shared memory per MMA (the build with four TMA producers).  For 3
         // and 4 rows (two core matrices of the dense planes) it measured 1-2 % faster but cost batch 2 3 %.
         if (p.M <= 2) {
-            if (handover == 0) {
-                HandoverSize alone;
-                alone.add(p.N, p.K, num_sms);
-                handover = alone.k_tiles();
-            }
-            if (handover == 4) return launch_umma_one<PolF8Long, 16>(p, num_sms, pdl, stream);
+            HandoverSize alone;
+            alone.add(p.N, p.K, num_sms);
+            if ((group != nullptr ? group : &alone)->k_tiles() == 4) return launch_umma_one<PolF8Long, 16>(p, num_sms, pdl, stream);
             return launch_umma_one<PolF8, 16>(p, num_sms, pdl, stream);
         }
         if (p.M <= 8) return launch_umma_one<PolF8, 32>(p, num_sms, pdl, stream);

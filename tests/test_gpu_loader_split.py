@@ -1,0 +1,48 @@
+"""The activations of the fp8-plane kernels, split by the product's own loaders or by the kernel in front of it: runs of k-tiles that
+cross the end of a row (also several times), ragged epochs, every input kind, both sides of the line.  Needs a B200."""
+import numpy as np
+import pytest
+import torch
+
+import decode_matmul_b200 as dmm
+from decode_matmul_b200 import _lib
+from oracle import dmm_oracle as o
+
+pytestmark = pytest.mark.gpu
+
+# Activations and weights are exact in the planes; what is left is the tensor core's accumulation, 8e-7 (relative 2-norm,
+# random terms) at any length, and the atomic adds of a few partial sums, 2^-24 each.
+REL = 1e-6
+
+
+def _inputs(kind, M, K, seed):
+    g = torch.Generator().manual_seed(seed)
+    if kind == "half":
+        x = torch.randn((M, K), generator=g).half()
+        return x, x.double(), dict(x_kind=_lib.X_F16)
+    if kind == "float":
+        x = torch.randn((M, K), generator=g)
+        return x, x.half().double(), dict(x_kind=_lib.X_F32)
+    x = torch.randn((M, 2 * K), generator=g)
+    return x, (torch.nn.functional.silu(x[:, :K]) * x[:, K:]).half().double(), dict(x_kind=_lib.X_F32_SILU_MUL, k=K, x_gap=K)
+
+
+# K = 32 and 96: a run of k-tiles crosses the end of the row at every (third) tile; 38400 and 37904 rows are 150 and 149 super-tiles,
+# one or two per CTA.  4096 x 1056: some three tiles per CTA, an epoch is never full.  9600 x 8192: 65 tiles per SM, where the
+# loaders split up to 6 rows and the kernel in front 7 and 8.
+@pytest.mark.parametrize("N,K", [(38400, 32), (37904, 96), (4096, 1056), (9600, 8192)])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 6, 7, 8])
+@pytest.mark.parametrize("kind", ["half", "float", "silu"])
+def test_split(kind, M, N, K):
+    rng = np.random.default_rng(N + K)
+    codes = rng.integers(-32768, 32768, size=(N, K // 8)).astype(np.int16)
+    cb16 = o.synthetic_codebook(42)
+    tiled, cb = torch.from_numpy(o.tile_pack(codes)).cuda(), torch.from_numpy(cb16).cuda()
+    w = dmm.decode_weights(tiled, cb).double()  # (bit-exact against the oracle: test_gpu_parity.py)
+    x, half, kw = _inputs(kind, M, K, M)
+    want = half.cuda() @ w.T
+    out = torch.zeros((M, N), device="cuda")
+    dmm.decode_matmul_fused(x.cuda(), tiled, cb, 1.0, out, accumulate=True, atomic=True, **kw)
+    # silu in the kernel uses the fast exponential: its rounding to half can differ by an ulp here and there
+    assert float((out.double() - want).norm() / want.norm()) <= (1e-4 if kind == "silu" else REL)
+    assert dmm.status() == 0
