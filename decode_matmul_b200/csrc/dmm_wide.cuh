@@ -32,15 +32,15 @@
 // Up to 64 columns there are two accumulator sets, so the next chain starts while the last one is read.
 //
 // Registers.  The compiler allocates 96 per thread, whatever setmaxnreg adds later, and the sums do not leave enough: -Xptxas -v
-// shows 144 bytes of spill stores and 80 of loads at 64 columns, 348 and 176 at 128 (fast layout 360 and 152), none at 32.  ncu
+// shows 144 bytes of spill stores and 48 of loads at 64 columns, 348 and 176 at 128 (fast layout 360 and 152), none at 32.  ncu
 // counts some five local loads and as many stores per warp and half unit at 128 columns (from 28672 x 8192 against x 16384),
 // those of the chains and epilogues included.
 //
 // Work split.  A tile of output is (256 rows, NB columns); its reduction is cut into units of 128 k.  While
 // there are more tiles than CTAs every CTA computes whole tiles; the units of the tiles that remain are
 // split evenly and contiguously over the CTAs (stream-K), partial tiles go through the workspace and
-// the last CTA to arrive (ticket) sums them in a fixed order, or straight into `out` with atomic adds
-// (DMM_FLAG_ATOMIC).  No CTA waits for another.  With too little workspace for the partials the remaining
+// the last CTA to arrive (ticket), or all of them together (share_fixup), sum them in a fixed order, or straight into
+// `out` with atomic adds (DMM_FLAG_ATOMIC).  No CTA depends on another being resident.  With too little workspace for the partials the remaining
 // tiles are computed whole.
 //
 // Warp roles (20 warps, 24 with kConv):
@@ -92,6 +92,7 @@ struct WideParams {
     int sst;            // super-tiles (256 output rows)
     int whole;          // whole tiles per CTA before the split ones
     int split_grid;     // CTAs that share the split tiles (0: none are left)
+    int share_fixup;    // 64-column build: the contributors of a split tile add up its parts together
     Part32 part;        // split units per CTA
     int stages;         // activation stages
     float *zero_ptr;    // optional: buffer this kernel clears on its way
@@ -191,6 +192,52 @@ struct WideWork {
         return s;
     }
 };
+
+// Fix-up of a split tile by all the CTAs that have a part of it (share_fixup).  Its ticket word counts, in three fields, the CTAs that
+// have written their part, the CTAs that have left, and the pieces (32 rows x 16 columns) that have been handed out: at
+// most 32, and one more per warp that asks, less than 2^12.  A CTA with nothing else to do stays until all parts are there, but
+// never longer than kWHelpCycles; then the warps of all CTAs that stayed take pieces until none is left and add up each in
+// the order of the contributors, so that the sums do not depend on who does it.  The last CTA to arrive never waits:
+// nothing depends on another CTA being resident.  The last one to leave clears the word.
+constexpr unsigned kWCountMask = 1023, kWLeftShift = 10, kWItemShift = 20;
+constexpr long long kWHelpCycles = 10000;
+// Shared where the parts of a tile are this many KiB or more; below the last CTA is done sooner by itself, the sharing costs
+// it some 1.5 us of atomics.  us, alone / shared: 64 x 4096 x 11008 (590 KiB) 26.5 / 22.8, 64 x 1024 x 28672 28.4 / 24.7, 56 x 5120 x 13824 27.2 /
+// 24.5, 64 x 4096 x 4096 16.8 / 14.3, 33 x 8192 x 8192 (220 KiB) 22.5 / 22.4.  Only in the 64-column build: up to 32
+// columns there is less to read (8 x 4096 x 4096 9.6 / 10.9), and at 128 the second form of the fix-up cost the kernel
+// registers (500 x 4096 x 4096 37.6 / 41.3).
+constexpr long long kWShareKiB = 150;
+
+// After the part has been written: flags[1] = all parts are there.
+__device__ __forceinline__ void fixup_arrive(unsigned *word, unsigned parts, bool stay, int tid, volatile int *flags) {
+    __threadfence();
+    named_barrier(1, kWDecWarps * 32);
+    if (tid == 0) {
+        bool all = ((atomicAdd(word, 1u) + 1u) & kWCountMask) == parts;
+        if (stay) {
+            const long long t0 = clock64();
+            while (!all && clock64() - t0 < kWHelpCycles) {
+                unsigned v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+                all = (v & kWCountMask) == parts;
+            }
+        }
+        flags[1] = all;
+    }
+    named_barrier(1, kWDecWarps * 32);
+}
+__device__ __forceinline__ int fixup_item(unsigned *word, int lane) {
+    unsigned got = 0;
+    if (lane == 0) got = atomicAdd(word, 1u << kWItemShift);
+    return static_cast<int>(__shfl_sync(0xffffffffu, got, 0) >> kWItemShift);
+}
+__device__ __forceinline__ void fixup_leave(unsigned *word, unsigned parts, int tid) {
+    named_barrier(1, kWDecWarps * 32);  // (flags[1] is reused by the next segment)
+    if (tid == 0) {
+        const unsigned old = atomicAdd(word, 1u << kWLeftShift);
+        if (((old >> kWLeftShift) & kWCountMask) == parts - 1u) *word = 0;
+    }
+}
 
 // Chains of one segment: its units cut into equal parts of at most kWChain.
 __device__ __forceinline__ int wide_chains(int units) { return (units + kWChain - 1) / kWChain; }
@@ -434,6 +481,58 @@ __global__ void __launch_bounds__(kConv ? kWConvThreads : kWThreads, 1) wide_ker
 #pragma unroll
                                 for (int e = 0; e < 16; ++e)
                                     if (b0 + e < mcols) __stcg(mine + (b0 + e) * 128, sum[g][e]);
+                            }
+                            if constexpr (kCols == 64) {
+                                if (p.share_fixup) {
+                                    const int a = prev.split * p.units;
+                                    const int c_lo = part32_owner(p.part, a), c_hi = part32_owner(p.part, a + p.units - 1);
+                                    const unsigned parts = static_cast<unsigned>(c_hi - c_lo + 1);
+                                    unsigned *const word = p.tickets + c_lo;
+                                    fixup_arrive(word, parts, ended == nseg - 1, tid, flags);
+                                    if (flags[1] != 0) {
+                                        __threadfence();
+                                        const int items = (mcols + 15) / 16 * 8;  // (16 columns, MMA tile, lane quarter)
+                                        for (;;) {
+                                            const int item = fixup_item(word, lane);
+                                            if (item >= items) break;
+                                            const int iq = item & 3, im = (item >> 2) & 1, b0 = (item >> 3) * 16;
+                                            float v[16];
+#pragma unroll
+                                            for (int e = 0; e < 16; ++e) v[e] = 0.f;
+                                            // fixed summation order; kFix contributors at a time
+                                            for (int c0 = c_lo; c0 <= c_hi; c0 += kFix) {
+                                                float l[kFix][16];
+#pragma unroll
+                                                for (int k = 0; k < kFix; ++k) {
+                                                    const int cc = c0 + k <= c_hi ? c0 + k : c_hi;
+                                                    const float *src = p.partials + (2ll * cc + (part32_begin(p.part, cc) > a ? 0 : 1)) * part_sz +
+                                                                       (static_cast<long long>(im) * p.nb + b0) * 128 + iq * 32 + lane;
+#pragma unroll
+                                                    for (int e = 0; e < 16; ++e)
+                                                        l[k][e] = b0 + e < mcols && c0 + k <= c_hi ? __ldcg(src + e * 128) : 0.f;
+                                                }
+#pragma unroll
+                                                for (int k = 0; k < kFix; ++k)
+#pragma unroll
+                                                    for (int e = 0; e < 16; ++e) v[e] += l[k][e];
+                                            }
+                                            const long long in = kFast ? static_cast<long long>(prev.ss) * 256 + 32 * (4 * im + iq) + lane
+                                                                       : (static_cast<long long>(prev.ss) * 16 + iq * 4 + (lane >> 3)) * 16 + 8 * im + (lane & 7);
+                                            if (in < p.N) {
+                                                float *const o = p.out + (m0 + b0) * p.N + in;
+#pragma unroll
+                                                for (int e = 0; e < 16; ++e)
+                                                    if (b0 + e < mcols) {
+                                                        const float r = v[e] * 32768.0f * p.scale;
+                                                        o[e * p.N] = p.accumulate ? o[e * p.N] + r : r;
+                                                    }
+                                            }
+                                        }
+                                    }
+                                    fixup_leave(word, parts, tid);
+                                    clear_sums();
+                                    continue;
+                                }
                             }
                             __threadfence();
                             named_barrier(1, kWDecWarps * 32);
@@ -768,18 +867,21 @@ inline int launch_wide(WideParams p, const void *x, int x_mode, long long x_ld, 
     const bool can_split = p.atomic_reduce || partial_capacity >= wide_partial_bytes(p.M, num_sms);
     if (rest > 0) {
         // How many CTAs share the remaining tiles: estimated cycles of the longest CTA.  A unit costs about
-        // 640 + 10 nb, and a split tile a fix-up: its last CTA reads nb KiB per contributor at 64 bytes a cycle.
+        // 640 + 10 nb, and a split tile a fix-up: its last CTA reads nb KiB per contributor at 64 bytes a cycle, or all of them
+        // about one part each.
         // (An estimate that ranks the splits well, not the rate: in the steady state a unit takes 1080 cycles up to 32
         // columns and 1480 at 128.)
         long long parts = rest, best = 0;
         for (long long c = rest; can_split && c <= num_sms; c = c < num_sms && c + rest > num_sms ? num_sms : c + rest) {
             if (c > rest && c > rest * p.units) break;
             const long long n = (rest * p.units + c - 1) / c, contributors = c == rest ? 0 : (c + rest - 1) / rest + 1;
-            const long long fix = contributors == 0 ? 0 : 3000 + 16 * p.nb * (p.atomic_reduce ? 1 : contributors + 1);
+            const bool share = !p.atomic_reduce && p.nb > 32 && p.nb <= 64 && p.nb * c >= kWShareKiB * rest;
+            const long long fix = contributors == 0 ? 0 : share ? 5000 + 32 * p.nb : 3000 + 16 * p.nb * (p.atomic_reduce ? 1 : contributors + 1);
             const long long cost = n * (640 + 10 * p.nb) + fix;
             if (best == 0 || cost < best) {
                 best = cost;
                 parts = c;
+                p.share_fixup = share ? 1 : 0;
             }
         }
         p.split_grid = static_cast<int>(parts);
