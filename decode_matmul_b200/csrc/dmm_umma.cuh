@@ -1494,24 +1494,25 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
                     // int8 activations go in as they are: a piece is 16 consecutive k of one row
                     const int8_t *x8 = reinterpret_cast<const int8_t *>(p.x);
                     const int nq = nt * 2 * M;
+                    // (all loads of a round first, at addresses that are always valid, and no divisions, as below: 32 x 28672 x 8192
+                    // 39.2 -> 33.0 us, 64 x 8192 x 8192 37.0 -> 32.9)
+                    const uint32_t inv = 65536u / static_cast<uint32_t>(2 * M) + 1u;
+                    const int kt_lo = (i0 + t_lo) % KT;
                     for (int pbase = 0; pbase < nq; pbase += LT * U) {
                         uint4 val[U];
                         uint32_t dst[U];
 #pragma unroll
                         for (int u = 0; u < U; ++u) {
-                            const int pc = pbase + u * LT + lt;
-                            dst[u] = 0;
-                            if (pc < nq) {
-                                const int jl = pc / (2 * M), rem = pc - jl * (2 * M), row = rem >> 1, kh = rem & 1;
-                                const int gt = i0 + t_lo + jl;
-                                const int kt = gt - (gt / KT) * KT;
-                                dst[u] = ebuf + jl * tile_b + kh * (tile_b / 2) + row * 16;
-                                val[u] = __ldcg(reinterpret_cast<const uint4 *>(x8 + static_cast<long long>(row) * p.x_ld + 32 * kt + 16 * kh));
-                            }
+                            const int pc = min(pbase + u * LT + lt, nq - 1);
+                            const int jl = static_cast<int>((static_cast<uint32_t>(pc) * inv) >> 16), rem = pc - jl * (2 * M), row = rem >> 1, kh = rem & 1;
+                            int kt = kt_lo + jl;
+                            while (kt >= KT) kt -= KT;
+                            dst[u] = ebuf + jl * tile_b + kh * (tile_b / 2) + row * 16;
+                            val[u] = __ldcg(reinterpret_cast<const uint4 *>(x8 + static_cast<long long>(row) * p.x_ld + 32 * kt + 16 * kh));
                         }
 #pragma unroll
                         for (int u = 0; u < U; ++u)
-                            if (dst[u] != 0) sts128(dst[u], val[u]);
+                            if (pbase + u * LT + lt < nq) sts128(dst[u], val[u]);
                     }
                 } else {
                     // Where a piece lies: the division by the pieces per tile as a multiplication (exact: an epoch has less than
