@@ -10,11 +10,11 @@ from oracle import dmm_oracle as o
 pytestmark = pytest.mark.gpu
 
 
-# M * N / 4 pieces of 16 bytes: fewer than a block has threads, one more than its threads, and more than the grid has
-@pytest.mark.parametrize("M,N", [(1, 16), (8, 128), (5, 208), (33, 1040), (65, 9488)])
+# Both ways of clearing: a memset below 32 tiles of 256 rows x 32 k per SM, a kernel from there on (9472 x 4096: 32 exactly, 37888 x 1056:
+# 33), with fewer and with more 16-byte pieces than the kernel has threads, and with two launches of the product.
+@pytest.mark.parametrize("M,N,K", [(1, 16, 96), (5, 208, 96), (65, 9488, 96), (8, 16, 32768), (1, 9472, 4096), (1, 37888, 1056), (33, 37888, 1056)])
 @pytest.mark.parametrize("pdl", [False, True])
-def test_result_that_held_something(M, N, pdl):
-    K = 96
+def test_result_that_held_something(M, N, K, pdl):
     rng = np.random.default_rng(M + N)
     cb = np.ascontiguousarray(o.build_codebook_abs())
     codes = rng.integers(-32768, 32768, size=(N, K // 8)).astype(np.int16)
