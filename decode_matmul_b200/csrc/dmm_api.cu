@@ -395,7 +395,7 @@ static int run_umma_i8(const void *x, const void *codes, const void *cb64, int32
     rc = resolve_workspace(d, M, K, workspace, workspace_bytes, stream, &ws);
     if (rc) return rc;
     // Integer sums do not depend on their order, so partial super-tiles are always added with
-    // atomics (no workspace round trip, no ticket); a plain product clears the output first (not counted as a launch).
+    // atomics (no workspace round trip, no ticket); a plain product clears the output first.
     bool pdl = (flags & DMM_FLAG_PDL) != 0;
     if (!(flags & DMM_FLAG_ACCUMULATE)) {
         // Small products are bound by what the host does, and there a memset is the cheaper call.  Per call, us, memset / kernel,
@@ -406,6 +406,7 @@ static int run_umma_i8(const void *x, const void *codes, const void *cb64, int32
             if (err != cudaSuccess) return err;
         } else {
             rc = launch_clear(out, static_cast<long long>(bytes), d->num_sms, pdl, stream);
+            g_launches.fetch_add(1, std::memory_order_relaxed);
             if (rc) return rc;
             pdl = true;  // the first product may start beside the clearing
         }
