@@ -1857,10 +1857,11 @@ inline int launch_umma_chain(const UmmaParams *ops, int n_ops, unsigned *sync, i
 // Whether the activations of a chunk of M <= 32 rows are split into planes once, by a kernel in front of the product, or by
 // the product's own loaders in every CTA.  The kernel in front is one more dependent launch, 2 to 3 us; the loaders' split
 // costs nothing up to 3 rows and then more with every row and tile, hence a number of tiles per SM for each row count.  us per
-// block of a stack, planes / loaders, and its products' mean tiles per SM: 4 rows 41.2 / 35.8 (42), 49.0 / 44.4 (65), 86.8 / 84.4 (176);
-// 5 rows 41.7 / 36.8, 49.3 / 45.8, 87.5 / 88.9; 6 rows 41.9 / 37.7, 49.5 / 48.3, 86.2 / 95.4; 7 rows 42.3 / 38.4, 50.0 / 50.4,
-// 88.3 / 102.0; 8 rows 42.6 / 40.4, 50.4 / 51.5, 88.9 / 108.8.  One product by itself: 4 rows 28672 x 8192 (194) 27.1 / 26.7, 8
-// rows 29.4 / 32.5.  The lines lie where straight lines through these meet.
+// block of a stack, planes / loaders, and its products' mean tiles per SM: 4 rows 41.2 / 34.7 (42), 49.0 / 42.5 (65), 86.8 / 83.1 (176);
+// 5 rows 41.7 / 35.2, 49.3 / 44.0, 87.5 / 86.9; 6 rows 41.9 / 36.2, 49.5 / 47.7, 86.2 / 94.5; 7 rows 42.3 / 37.4, 50.0 / 49.0,
+// 88.3 / 101.5; 8 rows 42.6 / 39.2, 50.4 / 51.0, 88.9 / 107.9.  One product by itself: 4 rows 28672 x 8192 (194) 27.1 / 26.7, 8
+// rows 29.4 / 32.5.  The lines lie where straight lines through these met before the loaders' first epoch grew; with it 5 and 7
+// rows would gain 1 to 2 % just beyond theirs.
 constexpr long long kPlanesMinBatch = 4;
 inline bool planes_in_front(long long M, long long tiles_per_sm) {
     constexpr int kMost[9] = {0, 0, 0, 0, 290, 144, 77, 63, 58};
