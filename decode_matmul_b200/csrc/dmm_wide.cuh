@@ -57,6 +57,7 @@
 //          zero_ptr.  A kernel that converts them beforehand costs a launch per product, more than this.
 // Every wait is bounded (mbar_wait).
 #pragma once
+#include "dmm_choice.h"
 #include "dmm_umma.cuh"
 
 namespace dmm {
@@ -201,12 +202,6 @@ struct WideWork {
 // nothing depends on another CTA being resident.  The last one to leave clears the word.
 constexpr unsigned kWCountMask = 1023, kWLeftShift = 10, kWItemShift = 20;
 constexpr long long kWHelpCycles = 10000;
-// Shared where the parts of a tile are this many KiB or more; below the last CTA is done sooner by itself, the sharing costs
-// it some 1.5 us of atomics.  us, alone / shared: 64 x 4096 x 11008 (590 KiB) 26.5 / 22.8, 64 x 1024 x 28672 28.4 / 24.7, 56 x 5120 x 13824 27.2 /
-// 24.5, 64 x 4096 x 4096 16.8 / 14.3, 33 x 8192 x 8192 (220 KiB) 22.5 / 22.4.  Only in the 64-column build: up to 32
-// columns there is less to read (8 x 4096 x 4096 9.6 / 10.9), and at 128 the second form of the fix-up cost the kernel
-// registers (500 x 4096 x 4096 37.6 / 41.3).
-constexpr long long kWShareKiB = 150;
 
 // After the part has been written: flags[1] = all parts are there.
 __device__ __forceinline__ void fixup_arrive(unsigned *word, unsigned parts, bool stay, int tid, volatile int *flags) {
@@ -866,24 +861,9 @@ inline int launch_wide(WideParams p, const void *x, int x_mode, long long x_ld, 
     long long grid = whole > 0 ? num_sms : 0;
     const bool can_split = p.atomic_reduce || partial_capacity >= wide_partial_bytes(p.M, num_sms);
     if (rest > 0) {
-        // How many CTAs share the remaining tiles: estimated cycles of the longest CTA.  A unit costs about
-        // 640 + 10 nb, and a split tile a fix-up: its last CTA reads nb KiB per contributor at 64 bytes a cycle, or all of them
-        // about one part each.
-        // (An estimate that ranks the splits well, not the rate: in the steady state a unit takes 1080 cycles up to 32
-        // columns and 1480 at 128.)
-        long long parts = rest, best = 0;
-        for (long long c = rest; can_split && c <= num_sms; c = c < num_sms && c + rest > num_sms ? num_sms : c + rest) {
-            if (c > rest && c > rest * p.units) break;
-            const long long n = (rest * p.units + c - 1) / c, contributors = c == rest ? 0 : (c + rest - 1) / rest + 1;
-            const bool share = !p.atomic_reduce && p.nb > 32 && p.nb <= 64 && p.nb * c >= kWShareKiB * rest;
-            const long long fix = contributors == 0 ? 0 : share ? 5000 + 32 * p.nb : 3000 + 16 * p.nb * (p.atomic_reduce ? 1 : contributors + 1);
-            const long long cost = n * (640 + 10 * p.nb) + fix;
-            if (best == 0 || cost < best) {
-                best = cost;
-                parts = c;
-                p.share_fixup = share ? 1 : 0;
-            }
-        }
+        const WideSplit split = wide_split(p.nb, p.units, rest, num_sms, can_split, p.atomic_reduce != 0);
+        const long long parts = split.parts;
+        p.share_fixup = split.share ? 1 : 0;
         p.split_grid = static_cast<int>(parts);
         if (!can_split) {  // one whole tile each
             p.part.a = p.units;
