@@ -318,8 +318,8 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
         p.M = M - m0 < step ? M - m0 : step;
         // (a consumer of the slots form splits what it sums up itself; the other tensor-parallel products keep one line)
         HandoverSize alone;
-        alone.add(N, K, d->num_sms);
-        if (f8 && (tp == nullptr ? planes_in_front(p.M, (group != nullptr ? group : &alone)->tiles_per_sm())
+        alone.add(N, K, d->num_sms, x_kind == DMM_X_F32_SILU_MUL);
+        if (f8 && (tp == nullptr ? planes_in_front(p.M, group != nullptr ? *group : alone)
                                  : tp->mode != 3 && p.M >= kPlanesMinBatch)) {
             // split the activations into E5M2 planes once, instead of once per CTA inside the kernel
             uint8_t *planes = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, d->num_sms);
@@ -910,7 +910,7 @@ int dmm_f16_sequence(const dmm_fused_op *ops, int n_ops, int64_t M, int sign_con
     if (current_device_state(&d) == 0)  // (else the first op says why not)
         for (int i = 0; i < n_ops; ++i)
             if (ops[i].N >= 16 && ops[i].N <= (1ll << 24) && ops[i].K >= 32 && ops[i].K <= (1ll << 17))  // (others will be refused)
-                size.add(ops[i].N, ops[i].K, d->num_sms);
+                size.add(ops[i].N, ops[i].K, d->num_sms, ops[i].x_kind == DMM_X_F32_SILU_MUL);
     for (int i = 0; i < n_ops; ++i) {
         const dmm_fused_op &op = ops[i];
         int rc = 0;

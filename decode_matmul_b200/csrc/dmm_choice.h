@@ -40,4 +40,43 @@ inline WideSplit wide_split(int nb, int units, long long rest, int num_sms, bool
     return s;
 }
 
+// Batch 1 and 2: four k-tiles per hand-over instead of two (PolF8Long) from 28 tiles per segment on.  The longer hand-over
+// gains with every tile and loses some 0.2 us at the end of each segment, where nothing is left to decode beside the MMAs
+// of the last one.  A CTA has about 1 + super-tiles / SMs segments.  PolF8 / PolF8Long in us, batch 1, added into a stack, and
+// tiles per segment: 57344 x 512 6.81 / 7.32 (10), 4096 x 4096 5.17 / 5.45 (13), 40960 x 1024 7.58 / 7.88 (17), 57344 x 1024 8.64 / 8.88
+// (19), 16384 x 2048 6.57 / 6.75 (19), 6144 x 6144 6.70 / 6.82 (27), 11008 x 4096 7.58 / 7.56 (29; a result of its own 10.93 / 10.82),
+// 57344 x 2048 13.14 / 13.13 (39), 8192 x 8192 9.11 / 9.00 (45), 28672 x 8192 20.6 / 20.1 (110).
+struct HandoverSize {
+    long long tiles = 0, segments = 0, sms = 0;  // of all CTAs; SMs of all products
+    long long silu_tiles = 0;                    // those of the products behind silu(gate) * up
+    void add(long long N, long long K, int num_sms, bool silu) {
+        const long long sst = (N + 255) / 256;
+        tiles += sst * (K / 32);
+        if (silu) silu_tiles += sst * (K / 32);
+        segments += sst + num_sms;
+        sms += num_sms;
+    }
+    int k_tiles() const { return tiles >= 28 * segments ? 4 : 2; }
+    long long tiles_per_sm() const { return tiles / sms; }
+};
+
+// Whether the activations of a chunk of M <= 32 rows are split into planes once, by a kernel in front of the product, or by
+// the product's own loaders in every CTA.  The kernel in front is one more dependent launch, 2 to 3 us; the loaders' split
+// costs nothing up to 3 rows and then more with every row and tile, hence a number of tiles per SM for each row count.  us per
+// block of a stack, planes / loaders, and its products' mean tiles per SM: 4 rows 41.2 / 34.7 (42), 49.0 / 42.5 (65), 86.8 / 83.1 (176);
+// 5 rows 41.7 / 35.2, 49.3 / 44.0, 87.5 / 86.9; 6 rows 41.9 / 36.2, 49.5 / 47.7, 86.2 / 94.5; 7 rows 42.3 / 37.4, 50.0 / 49.0,
+// 88.3 / 101.5; 8 rows 42.6 / 39.2, 50.4 / 51.0, 88.9 / 107.9.  The lines lie where straight lines through these met before the loaders'
+// first epoch grew.  One plain product by itself still gains at its line, us, fp32 activations: 4 rows 43008 x 8192 (290) 31.2 / 30.5, 5 rows 20480 x
+// 8192 (138) 18.1 / 17.1, 6 rows 11264 x 8192 (76) 13.0 / 12.1, 8 rows 8448 x 8192 (57) 11.7 / 11.1.
+// Behind silu(gate) * up the loaders of every super-tile repeat the exponential, and what is one product of four in a block decides
+// by itself: us per product, planes / loaders, launched programmatically 4 rows t = 41 10.3 / 9.6, 110 15.7 / 15.6, 290 32.2 / 34.8, 5 rows t = 138 18.2 / 20.3,
+// 8 rows t = 37 10.3 / 10.4, 57 11.7 / 13.1; one after the other 4 rows t = 27 10.1 / 9.7, 55 12.5 / 12.7, 110 16.9 / 17.6, 6 rows t = 13 9.1 / 7.9, 20 9.9 / 10.2, 8 rows
+// t = 20 10.1 / 10.5.  The lines are those at which neither way loses.
+constexpr long long kPlanesMinBatch = 4;
+inline bool planes_in_front(long long M, const HandoverSize &size) {
+    constexpr int kMost[9] = {0, 0, 0, 0, 290, 144, 77, 63, 58}, kMostSilu[9] = {0, 0, 0, 0, 40, 16, 16, 16, 16};
+    if (M < kPlanesMinBatch || M > 8) return M > 8;
+    return size.tiles_per_sm() > (2 * size.silu_tiles > size.tiles ? kMostSilu : kMost)[M];
+}
+
 }  // namespace dmm

@@ -57,6 +57,7 @@
 #include <functional>
 #include <type_traits>
 #include <unordered_map>
+#include "dmm_choice.h"
 #include "dmm_common.cuh"
 #include "dmm_launch.h"
 
@@ -1854,20 +1855,6 @@ inline int launch_umma_chain(const UmmaParams *ops, int n_ops, unsigned *sync, i
     return launch_umma_ops<PolF8, 32, true>(ops, n_ops, sync, num_sms, pdl, stream);
 }
 
-// Whether the activations of a chunk of M <= 32 rows are split into planes once, by a kernel in front of the product, or by
-// the product's own loaders in every CTA.  The kernel in front is one more dependent launch, 2 to 3 us; the loaders' split
-// costs nothing up to 3 rows and then more with every row and tile, hence a number of tiles per SM for each row count.  us per
-// block of a stack, planes / loaders, and its products' mean tiles per SM: 4 rows 41.2 / 34.7 (42), 49.0 / 42.5 (65), 86.8 / 83.1 (176);
-// 5 rows 41.7 / 35.2, 49.3 / 44.0, 87.5 / 86.9; 6 rows 41.9 / 36.2, 49.5 / 47.7, 86.2 / 94.5; 7 rows 42.3 / 37.4, 50.0 / 49.0,
-// 88.3 / 101.5; 8 rows 42.6 / 39.2, 50.4 / 51.0, 88.9 / 107.9.  One product by itself: 4 rows 28672 x 8192 (194) 27.1 / 26.7, 8
-// rows 29.4 / 32.5.  The lines lie where straight lines through these met before the loaders' first epoch grew; with it 5 and 7
-// rows would gain 1 to 2 % just beyond theirs.
-constexpr long long kPlanesMinBatch = 4;
-inline bool planes_in_front(long long M, long long tiles_per_sm) {
-    constexpr int kMost[9] = {0, 0, 0, 0, 290, 144, 77, 63, 58};
-    return M > 8 || (M >= kPlanesMinBatch && tiles_per_sm > kMost[M]);
-}
-
 // Padded batch rows of the plane layout for a batch of M (<= 32) rows.
 inline int planes_rows(long long M) { return M <= 8 ? static_cast<int>(M) : (M <= 16 ? 16 : 32); }
 
@@ -1920,24 +1907,6 @@ inline int launch_umma_i8(const UmmaParams &p, int num_sms, bool pdl, cudaStream
     return launch_umma_one<PolI8, 32>(p, num_sms, pdl, stream);
 }
 
-// Batch 1 and 2: four k-tiles per hand-over instead of two (PolF8Long) from 28 tiles per segment on.  The longer hand-over
-// gains with every tile and loses some 0.2 us at the end of each segment, where nothing is left to decode beside the MMAs
-// of the last one.  A CTA has about 1 + super-tiles / SMs segments.  PolF8 / PolF8Long in us, batch 1, added into a stack, and
-// tiles per segment: 57344 x 512 6.81 / 7.32 (10), 4096 x 4096 5.17 / 5.45 (13), 40960 x 1024 7.58 / 7.88 (17), 57344 x 1024 8.64 / 8.88
-// (19), 16384 x 2048 6.57 / 6.75 (19), 6144 x 6144 6.70 / 6.82 (27), 11008 x 4096 7.58 / 7.56 (29; a result of its own 10.93 / 10.82),
-// 57344 x 2048 13.14 / 13.13 (39), 8192 x 8192 9.11 / 9.00 (45), 28672 x 8192 20.6 / 20.1 (110).
-struct HandoverSize {
-    long long tiles = 0, segments = 0, sms = 0;  // of all CTAs; SMs of all products
-    void add(long long N, long long K, int num_sms) {
-        const long long sst = (N + 255) / 256;
-        tiles += sst * (K / 32);
-        segments += sst + num_sms;
-        sms += num_sms;
-    }
-    int k_tiles() const { return tiles >= 28 * segments ? 4 : 2; }
-    long long tiles_per_sm() const { return tiles / sms; }
-};
-
 // f8 != 0: PolF8 (needs M <= 32); else PolF16 with M <= 64.  group: the products that share one choice of the hand-over, null for
 // this product alone.
 inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cudaStream_t stream, const HandoverSize *group = nullptr) {
@@ -1952,7 +1921,7 @@ inline int launch_umma(bool f8, const UmmaParams &p, int num_sms, bool pdl, cuda
         // and 4 rows (two core matrices of the dense planes) it measured 1-2 % faster but cost batch 2 3 %.
         if (p.M <= 2) {
             HandoverSize alone;
-            alone.add(p.N, p.K, num_sms);
+            alone.add(p.N, p.K, num_sms, p.x_mode == kXSiluMul);
             if ((group != nullptr ? group : &alone)->k_tiles() == 4) return launch_umma_one<PolF8Long, 16>(p, num_sms, pdl, stream);
             return launch_umma_one<PolF8, 16>(p, num_sms, pdl, stream);
         }

@@ -15,6 +15,11 @@ extern "C" void wide(int nb, int units, long long rest, int sms, int can_split, 
     out[0] = s.parts;
     out[1] = s.share;
 }
+extern "C" int planes(long long M, int n, const long long *N, const long long *K, const int *silu, int sms) {
+    dmm::HandoverSize size;
+    for (int i = 0; i < n; ++i) size.add(N[i], K[i], sms, silu[i] != 0);
+    return dmm::planes_in_front(M, size);
+}
 """
 
 
@@ -52,3 +57,37 @@ def test_a_wide_split_stays_in_range(rules, nb):
                 assert tiles <= parts <= max(tiles, min(SMS, tiles * units))
                 assert share == (parts > tiles and not atomic and 32 < nb <= 64 and nb * parts >= 150 * tiles)
             assert _wide(rules, nb, units, tiles, can_split=False) == (tiles, False)
+
+
+def _planes(rules, M, *products):
+    n = len(products)
+    N, K = (ctypes.c_longlong * n)(*[p[0] for p in products]), (ctypes.c_longlong * n)(*[p[1] for p in products])
+    return bool(rules.planes(ctypes.c_longlong(M), n, N, K, (ctypes.c_int * n)(*[p[2] for p in products]), SMS))
+
+
+def _block(hidden, kv, ffn):
+    return (hidden + 2 * kv, hidden, 0), (hidden, hidden, 0), (2 * ffn, hidden, 0), (hidden, ffn, 1)
+
+
+# One product by itself behind silu(gate) * up: the loaders' exponential costs more than the planes kernel long before the line
+# of plain products.  N = 64 * SMS, K = 128 * t: t tiles per SM.
+@pytest.mark.parametrize("M,plain,silu", [(4, 290, 40), (5, 144, 16), (6, 77, 16), (7, 63, 16), (8, 58, 16)])
+def test_planes_in_front_of_one_product(rules, M, plain, silu):
+    for t, kind in ((plain, 0), (silu, 1)):
+        assert not _planes(rules, M, (64 * SMS, 128 * t, kind))
+        assert _planes(rules, M, (64 * SMS, 128 * (t + 1), kind))
+        assert not _planes(rules, M, *[(64 * SMS, 128 * t, kind)] * 4)
+        assert _planes(rules, M, *[(64 * SMS, 128 * (t + 1), kind)] * 4)
+
+
+# The blocks of a stack keep one choice, the plain lines: one product of four is behind silu.
+@pytest.mark.parametrize("M,shape,planes", [(4, (8192, 1024, 28672), False), (5, (4096, 4096, 11008), False), (5, (8192, 1024, 28672), True),
+                                            (8, (4096, 4096, 11008), False), (8, (5120, 5120, 13824), True)])
+def test_planes_in_front_of_a_block(rules, M, shape, planes):
+    assert _planes(rules, M, *_block(*shape)) == planes
+
+
+def test_planes_by_rows_alone(rules):
+    for kind in (0, 1):
+        assert not any(_planes(rules, M, (57344, 8192, kind)) for M in (1, 2, 3))
+        assert all(_planes(rules, M, (16, 32, kind)) for M in (9, 16, 17, 32))
