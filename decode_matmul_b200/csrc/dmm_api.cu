@@ -316,11 +316,9 @@ static int run_umma(bool f8, const void *x, int x_kind, long long x_ld, long lon
         UmmaParams p = {};
         p.x = reinterpret_cast<const uint8_t *>(x) + static_cast<size_t>(m0) * x_ld * (x_kind == DMM_X_F16 ? 2 : 4);
         p.M = M - m0 < step ? M - m0 : step;
-        // (a consumer of the slots form splits what it sums up itself; the other tensor-parallel products keep one line)
         HandoverSize alone;
         alone.add(N, K, d->num_sms, x_kind == DMM_X_F32_SILU_MUL);
-        if (f8 && (tp == nullptr ? planes_in_front(p.M, group != nullptr ? *group : alone)
-                                 : tp->mode != 3 && p.M >= kPlanesMinBatch)) {
+        if (f8 && (tp == nullptr ? planes_in_front(p.M, group != nullptr ? *group : alone) : planes_in_front_tp(p.M, tp->mode, alone))) {
             // split the activations into E5M2 planes once, instead of once per CTA inside the kernel
             uint8_t *planes = reinterpret_cast<uint8_t *>(ws) + planes_offset(M, d->num_sms);
             rc = launch_planes(p.x, x_kind, x_ld, x_gap, static_cast<int>(p.M), K, planes, pdl, stream);

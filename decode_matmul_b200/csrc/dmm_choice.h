@@ -73,10 +73,20 @@ struct HandoverSize {
 // 8 rows t = 37 10.3 / 10.4, 57 11.7 / 13.1; one after the other 4 rows t = 27 10.1 / 9.7, 55 12.5 / 12.7, 110 16.9 / 17.6, 6 rows t = 13 9.1 / 7.9, 20 9.9 / 10.2, 8 rows
 // t = 20 10.1 / 10.5.  The lines are those at which neither way loses.
 constexpr long long kPlanesMinBatch = 4;
+constexpr int kPlanesMost[9] = {0, 0, 0, 0, 290, 144, 77, 63, 58}, kPlanesMostSilu[9] = {0, 0, 0, 0, 40, 16, 16, 16, 16};
 inline bool planes_in_front(long long M, const HandoverSize &size) {
-    constexpr int kMost[9] = {0, 0, 0, 0, 290, 144, 77, 63, 58}, kMostSilu[9] = {0, 0, 0, 0, 40, 16, 16, 16, 16};
     if (M < kPlanesMinBatch || M > 8) return M > 8;
-    return size.tiles_per_sm() > (2 * size.silu_tiles > size.tiles ? kMostSilu : kMost)[M];
+    return size.tiles_per_sm() > (2 * size.silu_tiles > size.tiles ? kPlanesMostSilu : kPlanesMost)[M];
+}
+
+// The same for the tensor-parallel products; mode as in UmmaParams.  A consumer of the slots form (3) splits what it sums up
+// itself, and the kernel of its build with planes in turn with the one without costs more than planes gain: its producer (2) keeps
+// to the plain lines whatever its input.  us per block in a group of one, planes from 4 rows on / so: 2048 wide 4 rows 43.6 / 36.5, 5 rows
+// 48.0 / 39.3, 8 rows 50.2 / 41.8, 4096 wide 8 rows 75.1 / 69.7, 8192 wide 4 rows 127.6 / 124.5, 8 rows 172.1 / 172.2 (before there were
+// two builds: 42.6, 46.1, 50.0, 76.8, 133.0, 177.7).  Products that add into every rank's buffer (0): planes from 4 rows on.
+inline bool planes_in_front_tp(long long M, int mode, const HandoverSize &alone) {
+    if (mode == 0) return M >= kPlanesMinBatch;
+    return mode == 2 && M >= kPlanesMinBatch && (M > 8 || alone.tiles_per_sm() > kPlanesMost[M]);
 }
 
 }  // namespace dmm

@@ -20,6 +20,11 @@ extern "C" int planes(long long M, int n, const long long *N, const long long *K
     for (int i = 0; i < n; ++i) size.add(N[i], K[i], sms, silu[i] != 0);
     return dmm::planes_in_front(M, size);
 }
+extern "C" int planes_tp(long long M, int mode, long long N, long long K, int silu, int sms) {
+    dmm::HandoverSize size;
+    size.add(N, K, sms, silu != 0);
+    return dmm::planes_in_front_tp(M, mode, size);
+}
 """
 
 
@@ -91,3 +96,19 @@ def test_planes_by_rows_alone(rules):
     for kind in (0, 1):
         assert not any(_planes(rules, M, (57344, 8192, kind)) for M in (1, 2, 3))
         assert all(_planes(rules, M, (16, 32, kind)) for M in (9, 16, 17, 32))
+
+
+# The consumer of the slots form (mode 3) never has planes; its producer (2) follows the plain lines; products that add into every
+# rank's buffer (0) have them from 4 rows on.
+@pytest.mark.parametrize("M", range(1, 9))
+def test_planes_in_front_of_tensor_parallel_products(rules, M):
+    line = {4: 290, 5: 144, 6: 77, 7: 63, 8: 58}.get(M)
+
+    def tp(mode, t, silu=0):
+        return bool(rules.planes_tp(ctypes.c_longlong(M), mode, ctypes.c_longlong(64 * SMS), ctypes.c_longlong(128 * t), silu, SMS))
+
+    for silu in (0, 1):
+        assert not tp(3, 1, silu) and not tp(3, 400, silu)
+        assert tp(0, 1, silu) == tp(0, 400, silu) == (M >= 4)
+        assert not tp(2, line or 400, silu)
+        assert line is None or tp(2, line + 1, silu)

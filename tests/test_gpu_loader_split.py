@@ -48,3 +48,26 @@ def test_split(kind, M, N, K):
     # silu in the kernel uses the fast exponential: its rounding to half can differ by an ulp here and there
     assert float((out.double() - want).norm() / want.norm()) <= (1e-4 if kind == "silu" else REL)
     assert dmm.status() == 0
+
+
+# The slots form of the tensor-parallel step in a group of one: rows 4 to 8, where producer and consumer both split in their loaders
+# (no launch besides the four products of a block and the last sum), and a down projection of 67 tiles per SM, beyond the line of 8 rows.
+@pytest.mark.parametrize("batch,hidden,ffn,extra", [(4, 2048, 5632, 0), (5, 1024, 2816, 0), (6, 2048, 5632, 0), (8, 2048, 5632, 0), (8, 5632, 14336, 1)])
+def test_slots_form(batch, hidden, ffn, extra):
+    from decode_matmul_b200.linear import LinearStack
+
+    cfg = dict(hidden=hidden, kv_heads=4, head_dim=128, ffn=ffn, layers=2)
+    cb = dmm.synthetic_codebook(42)
+    plain = LinearStack(cfg, cb, "cuda", logical_seed=12, scale=2.0 ** -9)
+    slots = LinearStack(cfg, cb, "cuda", logical_seed=12, scale=2.0 ** -9, tp_mode="slots")
+    torch.manual_seed(batch)
+    for step in range(3):  # the epoch counter and the slot parities carry over
+        h0 = torch.randn(batch, hidden, device="cuda")
+        want = plain.step(h0.clone(), fused=True)
+        before = dmm.launch_count()
+        got = slots.step(h0.clone(), fused=True)
+        if step > 0 and torch.cuda.get_device_properties(0).multi_processor_count == 148:
+            assert dmm.launch_count() - before == (4 + extra) * cfg["layers"] + 1
+        assert dmm.status() == 0
+        # an activation whose sum comes out one bit lower can round to another half: as for the form at 1 and 3 rows
+        assert torch.allclose(got, want, rtol=2e-3, atol=2e-3), f"step {step}: {float((got - want).abs().max())}"
