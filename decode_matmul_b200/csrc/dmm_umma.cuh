@@ -262,16 +262,18 @@ constexpr int kFirstEpoch = 16;  // k-tiles in the first activation epoch of a C
 constexpr int kMaxEpoch = 48;    // and at most this many in the later ones: short epochs keep the
                                  // loaders' latency per epoch below the time the previous one lasts
 
-// k-tiles of the first epoch: nothing can be multiplied before it is staged.  split: the loaders split the activations (4 * M pieces
-// per tile), else they only copy.
-__host__ __device__ inline int first_epoch_tiles(int E, int M, int ntiles, bool split) {
+// k-tiles of the first epoch: nothing can be multiplied before it is staged.  longer: the loaders split the activations (4 * M pieces
+// per tile) and the results are added with atomics.
+__host__ __device__ inline int first_epoch_tiles(int E, int M, int ntiles, bool longer) {
     // Batch 1 with a long tile sequence: 8 measured better than 16, 4 and 2; short sequences: one epoch of 16.  Splitting from 3 rows on
     // 32 / M, one round of a loader team with two pieces per thread: a block of the 4096-wide stack 33.0 us at 3 rows, 34.7 at 4, 36.3 at
     // 6 (16 / M: 35.2, 35.8, 37.7; 64 / M the same or slower).  At 2 rows that only pays in long sequences: 8192 wide 74.6 -> 73.7, but 2048
-    // wide 18.9 -> 19.2.  Copies gain nothing from a longer first epoch (6 rows 8192 wide 87.7 -> 88.2).
+    // wide 18.9 -> 19.2.  Copies gain nothing from a longer first epoch (6 rows 8192 wide 87.7 -> 88.2), and results of their own lose where a CTA
+    // then reaches the end of its first super-tile last and does its fix-up in the middle of its work (5 rows 8192 x 3072 14.0 -> 16.5, 8 rows
+    // 15.9 -> 18.5, though 6 rows 4096 x 4096 16.7 -> 16.0).
     int e0 = (kFirstEpoch / M) & ~1;
     if (M == 1 && ntiles >= 64) e0 = kFirstEpoch / 2;
-    if (split && (M >= 3 || (M == 2 && ntiles >= 32))) e0 = (2 * kFirstEpoch / M) & ~1;
+    if (longer && (M >= 3 || (M == 2 && ntiles >= 32))) e0 = (2 * kFirstEpoch / M) & ~1;
     if (e0 < 2) e0 = 2;
     return e0 < E ? e0 : E;
 }
@@ -1054,22 +1056,25 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
 #pragma unroll
                             for (int b = 0; b < NB; ++b)
                                 if (b < p.M) {
-                                    // fixed summation order; eight loads in flight at a time
+                                    // Fixed summation order; eight loads in flight at a time.  Where the loaders split, the loads go to
+                                    // addresses that are always valid: with a branch around each that build had fewer in flight
+                                    // (8 rows 1024 x 4096 29.2 -> 27.4 us, 4096 x 4096 17.9 -> 17.4, 3 rows 4096 x 4096 13.3 -> 12.9).  With
+                                    // planes, where there are registers left, the branches are faster (8 rows 8192 x 4096 15.3 against 16.5).
                                     Acc tot = Acc(0);
                                     for (int c0 = 0; c0 < ncta; c0 += 8) {
                                         Acc part[8];
 #pragma unroll
                                         for (int e = 0; e < 8; ++e) {
                                             part[e] = Acc(0);
-                                            if (c0 + e < ncta) {
-                                                const int c = c_lo + c0 + e;
+                                            if (!kPlanes || c0 + e < ncta) {
+                                                const int c = min(c_lo + c0 + e, c_hi);
                                                 const int slot_c = part32_begin(p.part, c) > ss_a ? 0 : 1;
                                                 part[e] = __ldcg(partials_acc + static_cast<long long>(c * 2 + slot_c) * Plan::kPartial +
                                                                  (q * NB + b) * 128 + trow);
                                             }
                                         }
 #pragma unroll
-                                        for (int e = 0; e < 8; ++e) tot += part[e];
+                                        for (int e = 0; e < 8; ++e) tot += c0 + e < ncta ? part[e] : Acc(0);
                                     }
                                     Acc *o = out_acc + b * p.N + n;
                                     const Acc r = acc_scaled(p.scale, tot);
@@ -1170,7 +1175,7 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
             // descriptor of activation stage 0; later stages and k-halves only move the address field
             const uint32_t tile_b = plane_tile_bytes<NMMA, Pol::kIsInt != 0>(static_cast<int>(p.M));  // fp8: bytes of one k-tile of planes
             const int E = epoch_tiles(Plan::kEpochBytes, tile_b);  // k-tiles per epoch
-            const int E0 = first_epoch_tiles(E, static_cast<int>(p.M), i1 - i0, Pol::kIsF8 && !Pol::kIsInt && !kPlanes);  // the first one is short
+            const int E0 = first_epoch_tiles(E, static_cast<int>(p.M), i1 - i0, Pol::kIsF8 && !Pol::kIsInt && !kPlanes && p.atomic_reduce != 0);  // the first one is short
             // fp8: a plane is one 8-row core matrix (rows past the batch overlap the next plane and
             // land in unused columns) or, for the 16-row layout, two of them
             const uint64_t xdesc0 = Pol::kIsF8 ? smem_desc(x_addr, tile_b / 2, (NMMA > 32 || Pol::kIsInt) ? 128u : tile_b / 8)
@@ -1451,7 +1456,7 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
             const int E = epoch_tiles(Plan::kEpochBytes, tile_b);
             // The first epoch is short: nothing can be multiplied before it is staged, and the
             // loaders may only start once the previous kernel of the stream has finished.
-            const int E0 = first_epoch_tiles(E, M, i1 - i0, Pol::kIsF8 && !Pol::kIsInt && !kPlanes);
+            const int E0 = first_epoch_tiles(E, M, i1 - i0, Pol::kIsF8 && !Pol::kIsInt && !kPlanes && p.atomic_reduce != 0);
             const int ntiles = i1 - i0;
             const int nep = ntiles <= 0 ? 0 : (ntiles <= E0 ? 1 : 1 + (ntiles - E0 + E - 1) / E);
             // two teams of loader warps fill alternate epochs, so that the global-memory latency

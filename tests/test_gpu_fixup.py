@@ -31,3 +31,26 @@ def test_split_tiles(M, N, K):
         # another shape in between, with its own split, on the same workspace
         dmm.decode_matmul_fp16(small, tiled[:16, :4].contiguous(), cb)
     assert dmm.status() == 0
+
+
+# The small-batch kernels' own fix-up, eight parts at a time: 5 to 6 parts per super-tile, 9 to 10, 18 to 19, 37 and all 148, loads beyond the
+# last part included (the workspace holds NaN where nothing was written); rows that the loaders split and, at 8 rows 9600 x 8192, planes.
+@pytest.mark.parametrize("N,K", [(8192, 3072), (4096, 4096), (2048, 2048), (1024, 4096), (16, 32768), (9600, 8192)])
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8])
+def test_split_super_tiles(M, N, K):
+    gen = torch.Generator(device="cuda").manual_seed(M + N + K)
+    codes = torch.randint(-32768, 32768, (N, K // 8), dtype=torch.int16, device="cuda", generator=gen)
+    cb = torch.from_numpy(o.synthetic_codebook(42)).cuda()
+    x = torch.randn((M, K), device="cuda", generator=gen)
+    want = x.half().double() @ dmm.decode_weights(codes, cb).double().T
+    ws = torch.full((dmm.workspace_bytes(M, N, K),), 255, dtype=torch.uint8, device="cuda")
+    ws[:1024] = 0  # the counters
+    got = []
+    for _ in range(2):
+        y = torch.full((M, N), float("nan"), device="cuda")
+        dmm.decode_matmul_fused(x, codes, cb, 1.0, y, workspace=ws)
+        # exact products, sums off by the truncation of the tensor core: 7e-7 to 9e-7 at any length
+        assert float((y.double() - want).norm() / want.norm()) <= 2e-6
+        got.append(y)
+    assert torch.equal(got[0], got[1])
+    assert dmm.status() == 0
