@@ -1058,23 +1058,25 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
                                 if (b < p.M) {
                                     // Fixed summation order; eight loads in flight at a time.  Where the loaders split, the loads go to
                                     // addresses that are always valid: with a branch around each that build had fewer in flight
-                                    // (8 rows 1024 x 4096 29.2 -> 27.4 us, 4096 x 4096 17.9 -> 17.4, 3 rows 4096 x 4096 13.3 -> 12.9).  With
-                                    // planes, where there are registers left, the branches are faster (8 rows 8192 x 4096 15.3 against 16.5).
+                                    // (8 rows 1024 x 4096 29.2 -> 27.4 us, 4096 x 4096 17.9 -> 17.4, 3 rows 4096 x 4096 13.3 -> 12.9).  The other
+                                    // builds are faster with the branches: with planes 8 rows 8192 x 4096 15.3 against 16.5, and the
+                                    // integer build, which only ever adds, 32 rows 262144 x 32 15.3 against 20.0.
+                                    constexpr bool kClamp = Pol::kIsF8 && !Pol::kIsInt && !kPlanes;
                                     Acc tot = Acc(0);
                                     for (int c0 = 0; c0 < ncta; c0 += 8) {
                                         Acc part[8];
 #pragma unroll
                                         for (int e = 0; e < 8; ++e) {
                                             part[e] = Acc(0);
-                                            if (!kPlanes || c0 + e < ncta) {
-                                                const int c = min(c_lo + c0 + e, c_hi);
+                                            if (kClamp || c0 + e < ncta) {
+                                                const int c = kClamp ? min(c_lo + c0 + e, c_hi) : c_lo + c0 + e;
                                                 const int slot_c = part32_begin(p.part, c) > ss_a ? 0 : 1;
                                                 part[e] = __ldcg(partials_acc + static_cast<long long>(c * 2 + slot_c) * Plan::kPartial +
                                                                  (q * NB + b) * 128 + trow);
                                             }
                                         }
 #pragma unroll
-                                        for (int e = 0; e < 8; ++e) tot += c0 + e < ncta ? part[e] : Acc(0);
+                                        for (int e = 0; e < 8; ++e) tot += !kClamp || c0 + e < ncta ? part[e] : Acc(0);
                                     }
                                     Acc *o = out_acc + b * p.N + n;
                                     const Acc r = acc_scaled(p.scale, tot);
