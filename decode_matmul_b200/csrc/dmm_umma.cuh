@@ -1512,11 +1512,12 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
                     // 39.2 -> 33.0 us, 64 x 8192 x 8192 37.0 -> 32.9)
                     const uint32_t inv = 65536u / static_cast<uint32_t>(2 * M) + 1u;
                     const int kt_lo = (i0 + t_lo) % KT;
-                    for (int pbase = 0; pbase < nq; pbase += LT * U) {
-                        uint4 val[U];
-                        uint32_t dst[U];
+                    auto copy = [&](auto uu, int pbase) {
+                        constexpr int UU = decltype(uu)::value;
+                        uint4 val[UU];
+                        uint32_t dst[UU];
 #pragma unroll
-                        for (int u = 0; u < U; ++u) {
+                        for (int u = 0; u < UU; ++u) {
                             const int pc = min(pbase + u * LT + lt, nq - 1);
                             const int jl = static_cast<int>((static_cast<uint32_t>(pc) * inv) >> 16), rem = pc - jl * (2 * M), row = rem >> 1, kh = rem & 1;
                             int kt = kt_lo + jl;
@@ -1525,8 +1526,14 @@ __global__ void __launch_bounds__(kSplit ? kUThreads : kUThreads - (kUTmaWarps -
                             val[u] = __ldcg(reinterpret_cast<const uint4 *>(x8 + static_cast<long long>(row) * p.x_ld + 32 * kt + 16 * kh));
                         }
 #pragma unroll
-                        for (int u = 0; u < U; ++u)
+                        for (int u = 0; u < UU; ++u)
                             if (pbase + u * LT + lt < nq) sts128(dst[u], val[u]);
+                    };
+                    // (one piece per thread where that is enough: with few rows, or few tiles, three of four loads were for nothing)
+                    if (nq <= LT) {
+                        copy(std::integral_constant<int, 1>{}, 0);
+                    } else {
+                        for (int pbase = 0; pbase < nq; pbase += LT * U) copy(std::integral_constant<int, U>{}, pbase);
                     }
                 } else {
                     // Where a piece lies: the division by the pieces per tile as a multiplication (exact: an epoch has less than

@@ -71,3 +71,19 @@ def test_slots_form(batch, hidden, ffn, extra):
         assert dmm.status() == 0
         # an activation whose sum comes out one bit lower can round to another half: as for the form at 1 and 3 rows
         assert torch.allclose(got, want, rtol=2e-3, atol=2e-3), f"step {step}: {float((got - want).abs().max())}"
+
+
+# The integer kernel's loaders copy one piece per thread where an epoch has no more than 64 of them, else four: few rows and few tiles,
+# runs of k-tiles that cross the end of a row, epochs of exactly 64 pieces (2 * tiles * rows) and of a few more.
+@pytest.mark.parametrize("N,K", [(37904, 96), (65536, 32), (4096, 1056), (16, 32768), (9600, 2080)])
+@pytest.mark.parametrize("M", [1, 2, 4, 8, 13, 16, 17, 32])
+def test_integer_loaders(M, N, K):
+    gen = torch.Generator(device="cuda").manual_seed(M + N + K)
+    codes = torch.randint(-32768, 32768, (N, K // 8), dtype=torch.int16, device="cuda", generator=gen)
+    cb = dmm.build_codebook_abs("cuda")
+    x = torch.randint(-128, 128, (M, K), dtype=torch.int8, device="cuda", generator=gen)
+    base = torch.randint(-1000, 1000, (M, N), dtype=torch.int32, device="cuda", generator=gen)
+    want = (x.double() @ dmm.decode_weights(codes, cb).double().T).to(torch.int32)  # (whole numbers below 2^53: exact)
+    assert torch.equal(dmm.decode_matmul_i8(x, codes, cb), want)
+    assert torch.equal(dmm.decode_matmul_i8(x, codes, cb, base.clone(), accumulate=True), base + want)
+    assert dmm.status() == 0
