@@ -164,7 +164,7 @@ def test_fp16_family_large_batch_and_accumulate(path):
     _check_f16(y.cpu().numpy(), base + o.decode_matmul_f16(x, codes, cb16, 0.125, o.SIGN_FAST))
 
 
-@pytest.mark.parametrize("M", [2, 4, 12, 20])  # split inside the kernel (M < 4) and by planes_kernel, all row paddings
+@pytest.mark.parametrize("M", [2, 4, 12, 20])  # split by the loaders (a matrix as small as this: up to 8 rows) and by planes_kernel
 def test_fp8_plane_split_is_exact_for_awkward_activations(M):
     """Subnormal, tiny, huge and all-mantissa-bits halves: the four E5M2 planes must add up exactly."""
     rng = np.random.default_rng(9)
@@ -182,6 +182,32 @@ def test_fp8_plane_split_is_exact_for_awkward_activations(M):
     scale = np.abs(want).max()
     assert np.abs(got - want).max() <= 2e-5 * scale + 1e-6   # fp8-operand MMA: fewer accumulator bits
     assert np.abs(got2 - want).max() <= 2e-6 * scale + 1e-6
+
+
+# Up to 8 rows planes_kernel packs the rows densely; it runs on large matrices only (from 145 tiles per SM on at 5 rows, 78 at 6, 64
+# at 7, 59 at 8), which have to be computed on the GPU: decode_weights is bit-exact (above).
+@pytest.mark.parametrize("M,N", [(5, 21760), (6, 21760), (7, 9600), (8, 9600)])
+@pytest.mark.parametrize("layout", ["tile", "fast"])
+def test_dense_planes_are_exact_for_awkward_activations(M, N, layout):
+    K = 8192
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    codes = torch.randint(-32768, 32768, (N, K // 8), dtype=torch.int16, device="cuda", generator=gen)
+    lay = dmm.LAYOUT_FAST if layout == "fast" else dmm.LAYOUT_TILE
+    cb = _dev(o.synthetic_codebook(42))
+    bits = torch.randint(0, 0x7C00, (M, K), dtype=torch.int16, device="cuda", generator=gen)  # every finite positive half
+    bits[1] |= -0x8000
+    bits[M - 1, ::2] = torch.randint(0, 0x0400, (K // 2,), dtype=torch.int16, device="cuda", generator=gen)  # subnormals
+    x = (bits.view(torch.float16).float() * 2.0 ** -10).half()
+    w = dmm.decode_weights(codes, cb, layout=lay)
+    want = torch.cat([x.double() @ part.double().T for part in w.split(8192)], dim=1)
+    before = dmm.launch_count()
+    y = dmm.decode_matmul_fp16(x, codes, cb, 1.0, path=dmm.PATH_TCGEN05_F8, layout=lay)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert dmm.launch_count() - before == 2, "planes_kernel and the product"
+    # a row of activations of one sign has partial sums that only grow: truncated fp32 sums, as at K = 512 above; a plane
+    # that is lost or in the wrong place is off by 2^-12 of the largest terms and more
+    for got, ref in zip(y.double(), want):
+        assert float((got - ref).abs().max()) <= 2e-5 * float(ref.abs().max()) + 1e-6
 
 
 def test_fp16_family_scale_e8p_and_linearity(e8p):
@@ -314,9 +340,8 @@ def test_linear_stack_fused_step_matches_unfused():
 
 @pytest.mark.parametrize("batch", [5, 16, 32])
 def test_linear_stack_fused_step_at_larger_batches(batch):
-    """From 4 batch rows on the fused step splits the activations with planes_kernel (fp32 and
-    SiLU inputs included) and switches to the 64- and 128-column MMA variants: same result as the
-    plain step."""
+    """At 5 rows of a small stack the loaders split the activations (fp32 and SiLU inputs included), at 16 the wide
+    kernel converts them itself and at 32 half_kernel does before it: same result as the plain step."""
     from decode_matmul_b200.linear import LinearStack
 
     cfg = dict(hidden=512, kv_heads=2, head_dim=64, ffn=1024, layers=2)
