@@ -79,14 +79,18 @@ static size_t planes_offset(long long M, int num_sms) {
     return (ticket_bytes(num_sms) + partial_bytes(M, num_sms) + 255) & ~static_cast<size_t>(255);
 }
 // Which kernel a product of the fp16 family runs on: the wide one (dmm_wide.cuh) or the fp8-plane kernels.  Per
-// tile of codes (256 rows x 32 k) and SM the wide kernel costs more up to some 32 rows, per call it costs less (no
-// planes kernel, a cheaper fix-up), so the line is a number of tiles per SM, t.  Microseconds on the GPU (CUDA graph over
-// several matrices, programmatic launches), planes / wide:
-//   own result   4 rows    t = 31 13.7 / 11.2, 37 14.3 / 14.6         6 rows    48 15.9 / 12.7, 55 16.2 / 17.0
-//                8 rows    t = 55 17.0 / 17.2 (K = 4096) and 17.9 / 17.4 (K = 8192), 96 21.0 / 23.1
-//                9 rows    t = 55 19.2 / 17.2, 96 22.7 / 23.1         12 rows   96 24.2 / 23.3, 138 28.9 / 28.9
-//                16 rows   t = 138 30.6 / 29.3, 193 34.8 / 36.5       from 17 rows on always (t = 387 at 17: 67 / 65)
+// tile of codes (256 rows x 32 k) and SM the wide kernel costs more up to some 32 rows, per call it costs less (a
+// cheaper fix-up, from 9 rows on no planes kernel), so the line is a number of tiles per SM, t.  Microseconds on the GPU (CUDA
+// graph over several matrices, programmatic launches), planes / wide:
+//   own result   4 rows    t = 13 11.7 / 8.7, 31 14.1 / 11.5 (K = 9216) and 12.4 / 11.0 (K = 4096), 37 14.9 / 14.9 (K = 11008) and 13.1 / 14.3
+//                6 rows    t = 48 17.2 / 16.8 (K = 14336) and 14.6 / 16.0 (K = 4096), 55 18.3 / 17.5 (K = 16384) and 15.8 / 16.7
+//                8 rows    t = 37 15.3 / 14.9, 55 17.0 / 16.9 (K = 4096), 17.1 / 17.2 (K = 8192) and 20.4 / 18.0 (K = 16384), 96 21.1 / 22.5
+//                9 rows    t = 55 19.7 / 17.3, 96 22.8 / 22.5         12 rows   96 23.8 / 22.7, 138 29.0 / 28.1
+//                16 rows   t = 138 31.2 / 28.5, 193 34.2 / 35.2       from 17 rows on always (t = 387 at 17: 67 / 65)
 //                (the planes step up at 9 rows, from 32 to 64 MMA columns: hence two lines)
+//                The lines up to 8 rows were drawn when a planes kernel ran in front of every one of these products.  Now the
+//                loaders split, and how many CTAs share a super-tile counts as much as t: beyond what the lines say the wide kernel would
+//                win at 3 rows 4096 x 4096 (10.9 / 8.7), the planes at 4 rows 8192 x 4096 (t = 27, 11.8 / 12.9) and 6 rows 11008 x 4096 (14.1 / 14.7).
 //   added into a stack, fp32 activations.  A block of the stack with this product on planes / wide:
 //                9 to 16 rows: the wide kernel's own loaders convert them and fall behind on large matrices, the earlier
 //                the fewer rows there are to gain from: 9 rows t = 47 72.5 / 72.1, 55 101.8 / 102.1, 58 59.5 / 61.4; 16
@@ -396,8 +400,11 @@ static int run_umma_i8(const void *x, const void *codes, const void *cb64, int32
     // atomics (no workspace round trip, no ticket); a plain product clears the output first.
     bool pdl = (flags & DMM_FLAG_PDL) != 0;
     if (!(flags & DMM_FLAG_ACCUMULATE)) {
-        // Small products are bound by what the host does, and there a memset is the cheaper call.  Per call, us, memset / kernel,
-        // by tiles per SM: 8 x 16 x 4096 (1) 11.9 / 13.3, 8 x 4096 x 4096 (13) 13.8 / 13.7, 16 x 8192 x 8192 (55) 17.5 / 16.4.
+        // Small products are bound by what the host does, and there a memset is the cheaper call.  us per call in a queue of
+        // calls, memset / kernel, by tiles per SM: 8 x 16 x 4096 (0) 11.9 / 13.3, 8 x 4096 x 4096 (13) 13.8 / 13.7, 1, 8 and 16 x 9472 x 4096 (32)
+        // 13.4 / 13.4, 13.4 / 13.4, 15.4 / 13.4, 1 and 8 x 14336 x 4096 (48) 15.4 / 13.5 both, 64 x 57344 x 768 (36) 38.0 / 34.4.  In a CUDA graph the
+        // kernel saves 0.3 us, 1.5 with programmatic launches (1 x 9472 x 4096 9.1 / 7.6); a call that is waited for by itself pays 0.3
+        // to 0.5 us for it up to 8 rows (8 x 9472 x 4096 26.9 / 27.3) and gains from 16 on (28.6 / 27.7).
         const size_t bytes = static_cast<size_t>(M) * static_cast<size_t>(N) * sizeof(int32_t);
         if ((N + 255) / 256 * (K / 32) / d->num_sms < 32) {
             const cudaError_t err = cudaMemsetAsync(out, 0, bytes, stream);

@@ -67,7 +67,8 @@ struct HandoverSize {
 // 5 rows 41.7 / 35.2, 49.3 / 44.0, 87.5 / 86.9; 6 rows 41.9 / 36.2, 49.5 / 47.7, 86.2 / 94.5; 7 rows 42.3 / 37.4, 50.0 / 49.0,
 // 88.3 / 101.5; 8 rows 42.6 / 39.2, 50.4 / 51.0, 88.9 / 107.9.  The lines lie where straight lines through these met before the loaders'
 // first epoch grew.  One plain product by itself still gains at its line, us, fp32 activations: 4 rows 43008 x 8192 (290) 31.2 / 30.5, 5 rows 20480 x
-// 8192 (138) 18.1 / 17.1, 6 rows 11264 x 8192 (76) 13.0 / 12.1, 8 rows 8448 x 8192 (57) 11.7 / 11.1.
+// 8192 (138) 18.1 / 17.1, 6 rows 11264 x 8192 (76) 13.0 / 12.1, 8 rows 8448 x 8192 (57) 11.7 / 11.1; launched one after the other, where
+// the kernel in front waits for nothing, it is level there: 32.4 / 32.7, 19.4 / 19.0, 14.2 / 14.3, 12.8 / 13.2.
 // Behind silu(gate) * up the loaders of every super-tile repeat the exponential, and what is one product of four in a block decides
 // by itself: us per product, planes / loaders, launched programmatically 4 rows t = 41 10.3 / 9.6, 110 15.7 / 15.6, 290 32.2 / 34.8, 5 rows t = 138 18.2 / 20.3,
 // 8 rows t = 37 10.3 / 10.4, 57 11.7 / 13.1; one after the other 4 rows t = 27 10.1 / 9.7, 55 12.5 / 12.7, 110 16.9 / 17.6, 6 rows t = 13 9.1 / 7.9, 20 9.9 / 10.2, 8 rows
